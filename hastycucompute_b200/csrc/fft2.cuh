@@ -668,19 +668,6 @@ __global__ void __launch_bounds__(Q* kCW, (Q * kCW > 320) ? 1 : pass2_min_blocks
     }
 }
 
-// (P, Q) for the lengths with a register kernel; {0, 0} for the generic kernel.
-inline void reg_split(int L, int* P, int* Q) {
-    switch (L) {
-        case 64: *P = 8; *Q = 8; return;
-        case 128: *P = 8; *Q = 16; return;
-        case 256: *P = 16; *Q = 16; return;
-        case 320: *P = 16; *Q = 20; return;
-        case 512: *P = 16; *Q = 32; return;
-        case 640: *P = 20; *Q = 32; return;
-        default: *P = 0; *Q = 0; return;
-    }
-}
-
 // Op::kHalfIO (optional, default 0): the HM shape every pass of this operator has.
 template <class Op, class = void>
 struct HalfIO {
@@ -769,15 +756,18 @@ int launch_pass2_pq(const Op& op, PassCfg c, size_t extra_bytes, cudaStream_t s,
     }
 }
 
-// Runs the register kernel when L has one, otherwise the generic shared-memory kernel.
-// `extra_per_row` is the kSenseReduce accumulator size per outer row (bytes).
+// Lengths with a register kernel of their own.
+inline bool own_register_kernel(int L) {
+    return L == 64 || L == 128 || L == 256 || L == 320 || L == 512 || L == 640;
+}
+
+// The register kernel where L has one, else the shared-memory kernel. `extra_per_row` is the
+// kSenseReduce accumulator size per outer row (bytes).
 template <class Op>
-int launch_fft_pass(const Op& op, const FftLen& f, int64_t A, int64_t E, int Lin, int in_shift, int Lout,
-                    int out_shift, int inverse, size_t extra_per_row, cudaStream_t s, const char* name) {
-    int P, Q;
-    reg_split(f.L, &P, &Q);
+int launch_wide_pass(const Op& op, const FftLen& f, int64_t A, int64_t E, int Lin, int in_shift, int Lout,
+                     int out_shift, int inverse, size_t extra_per_row, cudaStream_t s, const char* name) {
     PassCfg c;
-    if (P > 0) {
+    if (own_register_kernel(f.L)) {
         pass_setup(&c, f, A, E, Lin, in_shift, Lout, out_shift, inverse, kCW);
         const size_t extra = extra_per_row * c.A_blk;
         switch (f.L) {

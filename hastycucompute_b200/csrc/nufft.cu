@@ -10,7 +10,7 @@
 #include <vector>
 
 #include "nufft.cuh"
-#include "ops.cuh"
+#include "modes_ops.cuh"
 
 namespace hb {
 
@@ -1025,98 +1025,6 @@ __global__ void __launch_bounds__(kGridThreads) k_interp_grad(const GridArgs a, 
         __syncwarp();
     }
 }
-
-// ---- x-axis passes between the caller's [C][N..] modes and the interleaved buffers ----------
-// Load modes f[e][a][l] (a = row over axes 0,1; l = axis 2) pre-scaled by 1/phihat.
-struct OpModesIn {
-    static constexpr bool kLoadLFast = true;
-    static constexpr bool kStoreLFast = false;
-    static constexpr bool kFusedK = false;
-    static constexpr bool kChunkLoop = false;
-    static constexpr bool kSenseReduce = false;
-    const float2* f;
-    float2* dst;  // [rows][nf2][C]
-    const float* d0;
-    const float* d1;
-    const float* d2;
-    int64_t N1, N2, nm;  // modes of axis 1, 2; modes per transform
-    int64_t d_a, d_l;
-    int64_t rows_f, fstride;  // frames: rows (N0 N1) and mode values (C nm) per frame; rows_f 0: one frame
-    __device__ __forceinline__ float2 load(int64_t a, int l, int64_t e) const {
-        // row a -> (frame, row of the frame) -> (mode 0, mode 1); 32-bit: F N0 N1 < 2^32 (setpts)
-        uint32_t al = (uint32_t)a;
-        int64_t fo = 0;
-        if (rows_f) {
-            const uint32_t fr = al / (uint32_t)rows_f;
-            al -= fr * (uint32_t)rows_f;
-            fo = (int64_t)fr * fstride;
-        }
-        const uint32_t i0 = al / (uint32_t)N1, i1 = al - i0 * (uint32_t)N1;
-        const float sc = d0[i0] * d1[i1] * d2[l];
-        return cscale(f[fo + e * nm + (int64_t)al * N2 + l], sc);
-    }
-    __device__ __forceinline__ int64_t kcol(int64_t) const { return 0; }
-    __device__ __forceinline__ const float2* kptr(int64_t) const { return nullptr; }
-    __device__ __forceinline__ const float2* srow(int64_t, int64_t) const { return nullptr; }
-    __device__ __forceinline__ float2 product_s(float2 v, float2) const { return v; }
-    __device__ __forceinline__ int64_t group(int64_t) const { return 0; }
-    __device__ __forceinline__ int ngroups() const { return 1; }
-    __device__ __forceinline__ float2 kval(int64_t, int, int64_t) const { return make_float2(0.f, 0.f); }
-    __device__ __forceinline__ void store(int64_t a, int o, int64_t e, float2 v) const { dst[a * d_a + (int64_t)o * d_l + e] = v; }
-    __device__ __forceinline__ float2 product(int64_t, int, int64_t, float2 v) const { return v; }
-    __device__ __forceinline__ void write_row(int64_t, int, int, float2) const {}
-    __device__ __forceinline__ void store_phase(const float2* res, const PassCfg& c, int64_t a0, int64_t e0, int, int,
-                                                float2*) const {
-        float2* d = dst;
-        const int64_t da = d_a, dl = d_l;
-        for_each_output<false>(res, c, a0, e0, [&](int64_t a, int o, int64_t e, float2 v) { d[a * da + (int64_t)o * dl + e] = v; });
-    }
-    __device__ __forceinline__ void finish(const PassCfg&, int64_t, float2*) const {}
-};
-
-// Store modes f[e][a][o] scaled by 1/phihat from the interleaved buffer.
-struct OpModesOut {
-    static constexpr bool kLoadLFast = false;
-    static constexpr bool kStoreLFast = true;
-    static constexpr bool kFusedK = false;
-    static constexpr bool kChunkLoop = false;
-    static constexpr bool kSenseReduce = false;
-    const float2* src;  // [rows][nf2][C]
-    float2* f;
-    const float* d0;
-    const float* d1;
-    const float* d2;
-    int64_t N1, N2, nm;
-    int64_t s_a, s_l;
-    int64_t rows_f, fstride;  // frames: rows (N0 N1) and mode values (C nm) per frame; rows_f 0: one frame
-    __device__ __forceinline__ float2 load(int64_t a, int l, int64_t e) const { return src[a * s_a + (int64_t)l * s_l + e]; }
-    __device__ __forceinline__ int64_t kcol(int64_t) const { return 0; }
-    __device__ __forceinline__ const float2* kptr(int64_t) const { return nullptr; }
-    __device__ __forceinline__ const float2* srow(int64_t, int64_t) const { return nullptr; }
-    __device__ __forceinline__ float2 product_s(float2 v, float2) const { return v; }
-    __device__ __forceinline__ int64_t group(int64_t) const { return 0; }
-    __device__ __forceinline__ int ngroups() const { return 1; }
-    __device__ __forceinline__ float2 kval(int64_t, int, int64_t) const { return make_float2(0.f, 0.f); }
-    __device__ __forceinline__ void store(int64_t a, int o, int64_t e, float2 v) const {
-        uint32_t al = (uint32_t)a;
-        int64_t fo = 0;
-        if (rows_f) {
-            const uint32_t fr = al / (uint32_t)rows_f;
-            al -= fr * (uint32_t)rows_f;
-            fo = (int64_t)fr * fstride;
-        }
-        const uint32_t i0 = al / (uint32_t)N1, i1 = al - i0 * (uint32_t)N1;
-        const float sc = d0[i0] * d1[i1] * d2[o];
-        f[fo + e * nm + (int64_t)al * N2 + o] = cscale(v, sc);
-    }
-    __device__ __forceinline__ float2 product(int64_t, int, int64_t, float2 v) const { return v; }
-    __device__ __forceinline__ void write_row(int64_t, int, int, float2) const {}
-    __device__ __forceinline__ void store_phase(const float2* res, const PassCfg& c, int64_t a0, int64_t e0, int, int,
-                                                float2*) const {
-        for_each_output<true>(res, c, a0, e0, [&](int64_t a, int o, int64_t e, float2 v) { store(a, o, e, v); });
-    }
-    __device__ __forceinline__ void finish(const PassCfg&, int64_t, float2*) const {}
-};
 
 // ---------------------------------------------------------------------------------------------
 // plan lifecycle

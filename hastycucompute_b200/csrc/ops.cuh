@@ -1,7 +1,7 @@
 // Pass operators shared by the NUFFT and Toeplitz paths (see fft.cuh for the Op contract).
 #pragma once
 
-#include "fft2.cuh"
+#include "fftp.cuh"
 
 namespace hb {
 
@@ -22,6 +22,17 @@ struct OpStrided {
     __device__ __forceinline__ float2 load(int64_t a, int l, int64_t e) const {
         return src[a * s_a + (int64_t)l * s_l + e];
     }
+    static constexpr int kPairShapes = 3;
+    // pair access (fftp.cuh)
+    bool vin_even() const { return ((s_a | s_l) & 1) == 0; }
+    const void* vin_base() const { return src; }
+    __device__ __forceinline__ const float2* vin(int64_t a, int64_t e) const { return src + a * s_a + e; }
+    __device__ __forceinline__ int64_t vin_l() const { return s_l; }
+    bool vout_even() const { return ((d_a | d_l) & 1) == 0; }
+    const void* vout_base() const { return dst; }
+    __device__ __forceinline__ float2* vout(int64_t a, int64_t e) const { return dst + a * d_a + e; }
+    __device__ __forceinline__ int64_t vout_l() const { return d_l; }
+    __device__ __forceinline__ c2 vout_value(c2 v) const { return {f2_mul(v.re, f2_dup(scale)), f2_mul(v.im, f2_dup(scale))}; }
     __device__ __forceinline__ int64_t kcol(int64_t) const { return 0; }
     __device__ __forceinline__ const float2* kptr(int64_t) const { return nullptr; }
     __device__ __forceinline__ const float2* srow(int64_t, int64_t) const { return nullptr; }
@@ -45,6 +56,8 @@ struct OpStrided {
     }
     __device__ __forceinline__ void finish(const PassCfg&, int64_t, float2*) const {}
 };
+
+HB_EXTERN_PASS(OpStrided)
 
 #endif
 
