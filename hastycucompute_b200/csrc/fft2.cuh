@@ -758,7 +758,7 @@ int launch_pass2_pq(const Op& op, PassCfg c, size_t extra_bytes, cudaStream_t s,
 
 // Lengths with a register kernel of their own.
 inline bool own_register_kernel(int L) {
-    return L == 64 || L == 128 || L == 256 || L == 320 || L == 512 || L == 640;
+    return L == 512 || L == 640;
 }
 
 // The register kernel where L has one, else the shared-memory kernel. `extra_per_row` is the
@@ -771,10 +771,6 @@ int launch_wide_pass(const Op& op, const FftLen& f, int64_t A, int64_t E, int Li
         pass_setup(&c, f, A, E, Lin, in_shift, Lout, out_shift, inverse, kCW);
         const size_t extra = extra_per_row * c.A_blk;
         switch (f.L) {
-            case 64: return launch_pass2_pq<8, 8>(op, c, extra, s, name);
-            case 128: return launch_pass2_pq<8, 16>(op, c, extra, s, name);
-            case 256: return launch_pass2_pq<16, 16>(op, c, extra, s, name);
-            case 320: return launch_pass2_pq<16, 20>(op, c, extra, s, name);
             case 512: return launch_pass2_pq<16, 32>(op, c, extra, s, name);
             case 640: return launch_pass2_pq<20, 32>(op, c, extra, s, name);
         }

@@ -269,14 +269,16 @@ constexpr bool pair_radix(int r) {
     return (r >= 8 && r <= 16) || r == 18 || r == 20 || r == 21 || r == 22 || r == 24 || r == 25 || r == 26;
 }
 
-// (P, Q) of length L, the most even split into two radices of the set (P even when that costs
-// nothing: a zero-padded input then skips half of step 1); {0, 0} where there is none.
-inline void pair_split(int L, int* P, int* Q) {
+// (P, Q) of length L, the most even split into two radices of the set; {0, 0} where there is none. Of the two
+// orders the one whose P (input_side) or Q is divisible by 4, else by 2: the side that a pass pads or crops.
+inline void pair_split(int L, bool input_side, int* P, int* Q) {
     *P = *Q = 0;
     for (int hi = 8; hi <= kRadixMax; ++hi) {
         if (!pair_radix(hi) || L % hi != 0 || L / hi > hi || !pair_radix(L / hi)) continue;
         const int lo = L / hi;
-        *P = lo % 2 == 0 ? lo : hi;
+        auto rank = [](int r) { return r % 4 == 0 ? 2 : r % 2 == 0 ? 1 : 0; };
+        const bool lo_first = input_side ? rank(lo) >= rank(hi) : rank(hi) >= rank(lo);
+        *P = lo_first ? lo : hi;
         *Q = L / *P;
         return;
     }
@@ -286,10 +288,11 @@ struct PairCfg {
     int P, Q, L;
     int Lin, in_shift;    // sample l -> position (l + in_shift) mod L, in_shift in [0, L)
     int Lout, out_shift;
+    int ph;               // centred input (1) / output (2): see pair_tw
     int vec_in, vec_out;  // pairs are 16-byte aligned neighbours
     int A_blk, E_blk;     // rows x inner columns per CTA (kSenseReduce: rows x inner pairs)
     int W;                 // columns of a job
-    int in_stride, in_elems, s_stride;
+    int in_stride, in_elems, s_stride, tw_n;
     int64_t n_jobs;
     int n_k;              // kFusedK: kernel columns staged in shared memory (0: read from global)
     unsigned n_eb;
@@ -297,6 +300,19 @@ struct PairCfg {
     const float2* tw;
 };
 
+
+// Operators of the NUFFT axes: kPairShapes bit 0 = the input has full length (type 1 crops), bit 1 = the
+// output has (type 2 pads). Where the other side is exactly half of it and centred, the pass runs the
+// shapes of a fixed half side (HM 2 / 1); otherwise HM 4 / 8 with a position check per element. Operators with
+// a fixed shape (kHalfIO) have that one.
+template <class Op, class = void>
+struct PairShapes {
+    static constexpr int value = 0;
+};
+template <class Op>
+struct PairShapes<Op, std::void_t<decltype(Op::kPairShapes)>> {
+    static constexpr int value = Op::kPairShapes;
+};
 
 // How a pass gets its samples into shared memory (cp.async, issued while the previous job is
 // transformed): an operator's columns lie side by side, sample (a, l, e) at vin(a, e) + l * vin_l(),
@@ -415,12 +431,25 @@ __device__ __forceinline__ void pair_fetch(const Op& op, const PairCfg& c, int P
     }
 }
 
+// Outer twiddle W_L^(t k1) of step 1. A centred half-length input (sample l at position l - L/4) is the
+// transform of the unshifted input times i^k, and a centred output is the unshifted output of the input times
+// i^n: with P (Q) divisible by 4 that is i^k1 (i^t), a quarter of the table added to the index
+// (the table then holds two periods). The pass itself pads and crops at offset 0.
+template <bool INV>
+__device__ __forceinline__ c2 pair_tw(const PairCfg& c, int L, int t, int k1, const float2* tw, c2 v) {
+    int at = t * k1;
+    if (c.ph & 1) at += ((3 * k1) & 3) * (L / 4);
+    if (c.ph & 2) at += ((3 * t) & 3) * (L / 4);
+    return c2_mul_tw<INV>(v, tw[at]);
+}
+
 // Step 1 for radix P: the thread's samples, P-point DFT, outer twiddles, into the transpose.
 template <int P, class Op, int HM, bool INV>
-__device__ __forceinline__ void pair_step1(const Op& op, const PairCfg& c, int Q, const PairCols& k, int t, int cp,
+__device__ __forceinline__ void pair_step1(const Op& op, const PairCfg& c, int L, int Q, const PairCols& k, int t, int cp,
                                            const float2* tw, const float4* In, c2* Y) {
     constexpr bool half = (HM & 1) != 0;
     constexpr bool prune = half && P % 2 == 0;
+    constexpr bool PH = PairShapes<Op>::value != 0 && (HM & 3) != 0;  // operators with centred sides
     c2 v[P];
     const c2 zero{0ull, 0ull};
     if constexpr (Op::kLoadLFast) {
@@ -442,7 +471,7 @@ __device__ __forceinline__ void pair_step1(const Op& op, const PairCfg& c, int Q
         c2_dft<P, INV>(v);
 #pragma unroll
     for (int k1 = 0; k1 < P; ++k1) {
-        if (k1 > 0) v[k1] = c2_mul_tw<INV>(v[k1], tw[t * k1]);
+        if (k1 > 0 || (PH && (c.ph & 2))) v[k1] = PH ? pair_tw<INV>(c, L, t, k1, tw, v[k1]) : c2_mul_tw<INV>(v[k1], tw[t * k1]);
         Y[pair_slot<Op>(k1 * Q + t, k1, cp)] = v[k1];
     }
 }
@@ -543,16 +572,16 @@ __global__ void __launch_bounds__((RMAX * kPairs + 31) / 32 * 32, MB) pair_kerne
     extern __shared__ float4 pair_smem[];
     c2* const Y = reinterpret_cast<c2*>(pair_smem);               // [L][kPairs]
     float4* const In = INPL ? pair_smem : pair_smem + L * kPairs;
-    float2* const tw = reinterpret_cast<float2*>(pair_smem + L * kPairs) + (INPL ? 0 : c.in_elems);  // [L]
-    float2* const Ks = tw + L;                                    // kFusedK: [n_k][L]
-    float2* const acc = tw + L;                                   // kSenseReduce: [Lout][kPairs] running sums
+    float2* const tw = reinterpret_cast<float2*>(pair_smem + L * kPairs) + (INPL ? 0 : c.in_elems);  // [tw_n]
+    float2* const Ks = tw + c.tw_n;                                  // kFusedK: [n_k][L]
+    float2* const acc = tw + c.tw_n;                                 // kSenseReduce: [Lout][kPairs] running sums
     float2* const Ss = acc + c.Lout * kPairs;                     // kSenseReduce: [kCW][s_stride] factor rows
     const int tid = threadIdx.x;
     const int cp = tid % kPairs, t = tid / kPairs;                // step 1 (and 3): t < Q
     const int cp2 = Op::kStoreLFast ? tid / P : cp;               // step 2: k1 < P
     const int k1 = Op::kStoreLFast ? tid - cp2 * P : t;
     const bool in1 = t < Q, in2 = Op::kStoreLFast ? cp2 < kPairs : k1 < P;
-    for (int i = tid; i < L; i += blockDim.x) cp_async8(tw + i, c.tw + i);
+    for (int i = tid; i < c.tw_n; i += blockDim.x) cp_async8(tw + i, c.tw + (i < L ? i : i - L));
 
     int64_t jq = blockIdx.x, ab = 0;
     unsigned eb = 0;
@@ -607,7 +636,7 @@ __global__ void __launch_bounds__((RMAX * kPairs + 31) / 32 * 32, MB) pair_kerne
         if (in1) {
             const PairCols k = pair_cols<Op>(c, a0, e0, cp);
             radix_switch<RMIN, RMAX, PT>(P, [&](auto rc) {
-                pair_step1<decltype(rc)::value, Op, HM, INV>(op, c, Q, k, t, cp, tw, In, Y);
+                pair_step1<decltype(rc)::value, Op, HM, INV>(op, c, L, Q, k, t, cp, tw, In, Y);
             });
         }
         if (Op::kFusedK || Op::kSenseReduce) cp_async_wait_all();
@@ -696,7 +725,8 @@ int launch_pair_inst(const Op& op, PairCfg c, cudaStream_t s, const char* name) 
     c.in_stride = c.Lin | 1;
     c.s_stride = c.Lout | 1;
     c.in_elems = Op::kLoadLFast ? (kCW * c.in_stride + 1) / 2 * 2 : c.Lin * kCW;
-    size_t smem = (size_t)c.L * kPairs * sizeof(c2) + (size_t)c.L * sizeof(float2);
+    c.tw_n = c.ph ? 2 * c.L : c.L;
+    size_t smem = (size_t)c.L * kPairs * sizeof(c2) + (size_t)c.tw_n * sizeof(float2);
     if (!INPL) smem += (size_t)c.in_elems * sizeof(float2);
     if (Op::kFusedK) smem += (size_t)c.n_k * c.L * sizeof(float2);
     if (Op::kSenseReduce) smem += (size_t)(c.Lout * kPairs + kCW * c.s_stride) * sizeof(float2);
@@ -719,6 +749,13 @@ int launch_pair_inst(const Op& op, PairCfg c, cudaStream_t s, const char* name) 
 template <class Op, int HM, bool INV>
 int launch_pair_dir(const Op& op, const PairCfg& c, cudaStream_t s, const char* name) {
     const int r = std::max(c.P, c.Q);
+    // the edges of the common matrix sizes have their radices as constants (the run-time switch costs 5 - 15 %)
+    if constexpr ((HM & 3) != 0) {
+        if (c.P == 8 && c.Q == 8) return launch_pair_inst<Op, HM, INV, 8, 8, 8, 8, 8>(op, c, s, name);
+        if (c.P == 8 && c.Q == 16) return launch_pair_inst<Op, HM, INV, 8, 16, 8, 16, 4>(op, c, s, name);
+        if (c.P == 16 && c.Q == 16) return launch_pair_inst<Op, HM, INV, 16, 16, 16, 16, 4>(op, c, s, name);
+        if (c.P == 16 && c.Q == 20) return launch_pair_inst<Op, HM, INV, 16, 20, 16, 20, 3>(op, c, s, name);
+    }
     if (r <= 16) return launch_pair_inst<Op, HM, INV, 8, 16, 0, 0, 4>(op, c, s, name);
     if (r <= 20) return launch_pair_inst<Op, HM, INV, 9, 20, 0, 0, 3>(op, c, s, name);
     return launch_pair_inst<Op, HM, INV, 10, kRadixMax, 0, 0, 2>(op, c, s, name);
@@ -726,27 +763,17 @@ int launch_pair_dir(const Op& op, const PairCfg& c, cudaStream_t s, const char* 
 
 inline bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
-// Operators whose fused type-1 / type-2 shapes the pair kernel is built for: kPairShapes bit 0 = full
-// input (crop), bit 1 = full output (pad); operators with a fixed shape (kHalfIO) have that one.
-template <class Op, class = void>
-struct PairShapes {
-    static constexpr int value = 0;
-};
+// Runs the pass on column pairs. *done is false where the length or the pass's shape has no instance.
 template <class Op>
-struct PairShapes<Op, std::void_t<decltype(Op::kPairShapes)>> {
-    static constexpr int value = Op::kPairShapes;
-};
-
-// Runs the pass on column pairs; P and Q are the split of f.L (pair_split). *done is false where the pass's
-// shape has no instance.
-template <class Op>
-int launch_pair_pass(const Op& op, const FftLen& f, int P, int Q, int64_t A, int64_t E, int Lin, int in_shift, int Lout,
+int launch_pair_pass(const Op& op, const FftLen& f, int64_t A, int64_t E, int Lin, int in_shift, int Lout,
                      int out_shift, int inverse, cudaStream_t s, const char* name, bool* done) {
     constexpr int HMop = HalfIO<Op>::value;
     PairCfg c{};
     const int L = f.L;
-    c.P = P;
-    c.Q = Q;
+    const bool crops = Lout < Lin;
+    pair_split(L, !crops, &c.P, &c.Q);
+    *done = c.P > 0;
+    if (!*done) return HB_OK;
     c.L = L;
     c.Lin = Lin;
     c.in_shift = ((in_shift % L) + L) % L;
@@ -755,7 +782,6 @@ int launch_pair_pass(const Op& op, const FftLen& f, int P, int Q, int64_t A, int
     c.A = A;
     c.E = E;
     c.tw = f.tw;
-    *done = true;
     const bool full_in = Lin == L && c.in_shift == 0, full_out = Lout == L && c.out_shift == 0;
     if (HMop != 0) {
         const bool ok_in = (HMop & 1) ? (2 * Lin == L && c.in_shift == 0) : full_in;
@@ -794,11 +820,22 @@ int launch_pair_pass(const Op& op, const FftLen& f, int P, int Q, int64_t A, int
     if constexpr (HMop != 0) {
         return launch_pair_dir<Op, HMop, (HMop & 3) == 2>(op, c, s, name);
     } else {
+        const int centred = L - L / 4;  // the shift -L/4
         if constexpr ((PairShapes<Op>::value & 1) != 0) {
+            if (full_in && 2 * Lout == L && c.out_shift == centred && L % 4 == 0 && c.Q % 4 == 0) {
+                c.out_shift = 0;
+                c.ph = 2;
+                return inverse ? launch_pair_dir<Op, 2, true>(op, c, s, name) : launch_pair_dir<Op, 2, false>(op, c, s, name);
+            }
             if (full_in && !full_out)
                 return inverse ? launch_pair_dir<Op, 4, true>(op, c, s, name) : launch_pair_dir<Op, 4, false>(op, c, s, name);
         }
         if constexpr ((PairShapes<Op>::value & 2) != 0) {
+            if (full_out && 2 * Lin == L && c.in_shift == centred && L % 4 == 0 && c.P % 4 == 0) {
+                c.in_shift = 0;
+                c.ph = 1;
+                return inverse ? launch_pair_dir<Op, 1, true>(op, c, s, name) : launch_pair_dir<Op, 1, false>(op, c, s, name);
+            }
             if (full_out && !full_in)
                 return inverse ? launch_pair_dir<Op, 8, true>(op, c, s, name) : launch_pair_dir<Op, 8, false>(op, c, s, name);
         }
@@ -813,13 +850,9 @@ int launch_pair_pass(const Op& op, const FftLen& f, int P, int Q, int64_t A, int
 template <class Op>
 int launch_fft_pass(const Op& op, const FftLen& f, int64_t A, int64_t E, int Lin, int in_shift, int Lout, int out_shift,
                     int inverse, size_t extra_per_row, cudaStream_t s, const char* name) {
-    int P = 0, Q = 0;
-    if (!own_register_kernel(f.L)) pair_split(f.L, &P, &Q);
-    if (P > 0) {
-        bool done = false;
-        const int st = launch_pair_pass(op, f, P, Q, A, E, Lin, in_shift, Lout, out_shift, inverse, s, name, &done);
-        if (st != HB_OK || done) return st;
-    }
+    bool done = false;
+    const int st = launch_pair_pass(op, f, A, E, Lin, in_shift, Lout, out_shift, inverse, s, name, &done);
+    if (st != HB_OK || done) return st;
     return launch_wide_pass(op, f, A, E, Lin, in_shift, Lout, out_shift, inverse, extra_per_row, s, name);
 }
 
