@@ -293,6 +293,7 @@ struct PairCfg {
     int A_blk, E_blk;     // rows x inner columns per CTA (kSenseReduce: rows x inner pairs)
     int W;                 // columns of a job
     int in_stride, in_elems, s_stride, tw_n;
+    int rows;              // kLoadLFast: the row factors are copied once per row
     int64_t n_jobs;
     int n_k;              // kFusedK: kernel columns staged in shared memory (0: read from global)
     unsigned n_eb;
@@ -319,12 +320,14 @@ struct PairShapes<Op, std::void_t<decltype(Op::kPairShapes)>> {
 // and go to In[l][kPairs] as pairs (16-byte copies where pairs are aligned neighbours); or (kLoadLFast)
 // each column is contiguous along l, at cin(a, e) + l, and goes to In[column][in_stride] (8-byte
 // copies, odd stride: step 1 then reads different banks), where cvalue applies the operator's factors.
+// kVecOut: a column's state is the address of output 0, outputs vout_l() apart, each through vout_value; a
+// pair is one 16-byte store where vec_out.
 template <class Op, class = void>
 struct HasVecOut {
     static constexpr bool value = false;
 };
 template <class Op>
-struct HasVecOut<Op, std::void_t<decltype(&Op::vout)>> {
+struct HasVecOut<Op, std::void_t<decltype(Op::kVecOut)>> {
     static constexpr bool value = true;
 };
 
@@ -399,7 +402,7 @@ __device__ __forceinline__ void pair_inputs(const PairCfg& c, int Q, int t, F&& 
 
 // Copies a job's samples into In (all threads).
 template <int HM, class Op>
-__device__ __forceinline__ void pair_fetch(const Op& op, const PairCfg& c, int P, int Q, int64_t a0, int64_t e0, float4* In) {
+__device__ __forceinline__ void pair_fetch(const Op& op, const PairCfg& c, int64_t a0, int64_t e0, float4* In, float2* Rs) {
     if constexpr (Op::kLoadLFast) {
         // a warp per column
         for (int col = threadIdx.x >> 5; col < c.W; col += blockDim.x >> 5) {
@@ -408,6 +411,12 @@ __device__ __forceinline__ void pair_fetch(const Op& op, const PairCfg& c, int P
             const float2* p = op.cin(a0 + al, e0 + el);
             float2* d = reinterpret_cast<float2*>(In) + col * c.in_stride;
             for (int l = threadIdx.x & 31; l < c.Lin; l += 32) cp_async8(d + l, p + l);
+        }
+        if (c.rows) {
+            for (int i = threadIdx.x; i < c.A_blk * c.Lin; i += blockDim.x) {
+                const int al = c.A_blk == 1 ? 0 : i / c.Lin, l = i - al * c.Lin;
+                if (a0 + al < c.A) cp_async8(Rs + i, op.row(a0 + al, e0) + l);
+            }
         }
     } else {
         const int cp = threadIdx.x % kPairs;
@@ -446,14 +455,18 @@ __device__ __forceinline__ c2 pair_tw(const PairCfg& c, int L, int t, int k1, co
 // Step 1 for radix P: the thread's samples, P-point DFT, outer twiddles, into the transpose.
 template <int P, class Op, int HM, bool INV>
 __device__ __forceinline__ void pair_step1(const Op& op, const PairCfg& c, int L, int Q, const PairCols& k, int t, int cp,
-                                           const float2* tw, const float4* In, c2* Y) {
+                                           const float2* tw, const float4* In, const float2* Rs, int64_t a0, c2* Y) {
     constexpr bool half = (HM & 1) != 0;
     constexpr bool prune = half && P % 2 == 0;
     constexpr bool PH = PairShapes<Op>::value != 0 && (HM & 3) != 0;  // operators with centred sides
     c2 v[P];
     const c2 zero{0ull, 0ull};
     if constexpr (Op::kLoadLFast) {
-        const auto f0 = op.cstate(k.a0, k.e0, k.ok0), f1 = op.cstate(k.a1, k.e1, k.ok1);
+        auto f0 = op.cstate(k.a0, k.e0, k.ok0), f1 = op.cstate(k.a1, k.e1, k.ok1);
+        if (c.rows) {  // the rows' factors were copied with the samples
+            op.cstate_row(f0, Rs + (k.ok0 ? (k.a0 - a0) * c.Lin : 0));
+            op.cstate_row(f1, Rs + (k.ok1 ? (k.a1 - a0) * c.Lin : 0));
+        }
         pair_inputs<P, HM>(c, Q, t, [&](int j, int l) {
             const float2* x = reinterpret_cast<const float2*>(In) + 2 * cp * c.in_stride + l;
             v[j] = c2_pack(k.ok0 ? op.cvalue(f0, l, x[0]) : make_float2(0.f, 0.f),
@@ -502,26 +515,36 @@ __device__ __forceinline__ void pair_outputs(const PairCfg& c, int P, int k1, F&
     }
 }
 
+// Where an operator's outputs of one column go: operators without vout give a column state (OState ostate(a, e),
+// computed once per column) and ostore(state, o, value).
 template <class Op>
-__device__ __forceinline__ void pair_store(const Op& op, const PairCfg& c, const PairCols& k, int o, c2 v) {
-    if constexpr (HasVecOut<Op>::value) {
-        if (c.vec_out) {
-            if (k.ok0) c2_st16(op.vout(k.a0, k.e0) + o * op.vout_l(), op.vout_value(v));
-            return;
+struct PairOut {
+    const Op& op;
+    const PairCfg& c;
+    const PairCols& k;
+    typename Op::OState s0, s1;
+    __device__ __forceinline__ PairOut(const Op& op_, const PairCfg& c_, const PairCols& k_)
+        : op(op_), c(c_), k(k_), s0(op_.ostate(k_.a0, k_.e0, k_.ok0)), s1(op_.ostate(k_.a1, k_.e1, k_.ok1)) {}
+    __device__ __forceinline__ void operator()(int o, c2 v) const {
+        if constexpr (HasVecOut<Op>::value) {
+            if (c.vec_out) {
+                if (k.ok0) c2_st16(s0 + o * op.vout_l(), op.vout_value(v));
+                return;
+            }
         }
+        float2 x0, x1;
+        c2_unpack(v, x0, x1);
+        if (k.ok0) op.ostore(s0, o, x0);
+        if (k.ok1) op.ostore(s1, o, x1);
     }
-    float2 x0, x1;
-    c2_unpack(v, x0, x1);
-    if (k.ok0) op.store(k.a0, o, k.e0, x0);
-    if (k.ok1) op.store(k.a1, o, k.e1, x1);
-}
+};
 
 // Fused kernel pass: multiply the spectrum u (positions k1 + P k2) by the kernel, inverse Q-point DFT,
 // inverse outer twiddles, back into the slots it came from.
 template <int Q, class Op>
 __device__ __forceinline__ void pair_kernel_mul(const Op& op, const PairCfg& c, int P, const PairCols& k, int k1, int cp,
                                                 const float2* tw, c2* Y, const float2* Ks, int64_t kc0, c2* u) {
-    const int64_t q0 = k.ok0 ? op.kcol(k.e0) : kc0, q1 = k.ok1 ? op.kcol(k.e1) : q0;
+    const int64_t q0 = k.ok0 ? op.kcol(k.e0) : c.n_k ? kc0 : 0, q1 = k.ok1 ? op.kcol(k.e1) : q0;
     const float2* w0 = c.n_k ? Ks + (q0 - kc0) * c.L : op.kptr(q0);
     const float2* w1 = c.n_k ? Ks + (q1 - kc0) * c.L : op.kptr(q1);
     if (q0 == q1) {
@@ -569,10 +592,13 @@ __device__ __forceinline__ void radix_switch(int r, F&& f) {
 template <class Op, int HM, bool INV, int RMIN, int RMAX, int PT, int QT, int MB, bool INPL>
 __global__ void __launch_bounds__((RMAX * kPairs + 31) / 32 * 32, MB) pair_kernel(const Op op, const PairCfg c) {
     const int P = PT ? PT : c.P, Q = QT ? QT : c.Q, L = PT ? PT * QT : c.L;
+    // in-place samples: the next job's copies go out between step 2's reads and stores, except where that spills
+    constexpr bool kEarly = PT != 0 && (HM & 4) == 0;
     extern __shared__ float4 pair_smem[];
     c2* const Y = reinterpret_cast<c2*>(pair_smem);               // [L][kPairs]
     float4* const In = INPL ? pair_smem : pair_smem + L * kPairs;
     float2* const tw = reinterpret_cast<float2*>(pair_smem + L * kPairs) + (INPL ? 0 : c.in_elems);  // [tw_n]
+    float2* const Rs = tw + c.tw_n;                               // rows: [A_blk][Lin] row factors
     float2* const Ks = tw + c.tw_n;                                  // kFusedK: [n_k][L]
     float2* const acc = tw + c.tw_n;                                 // kSenseReduce: [Lout][kPairs] running sums
     float2* const Ss = acc + c.Lout * kPairs;                     // kSenseReduce: [kCW][s_stride] factor rows
@@ -595,31 +621,14 @@ __global__ void __launch_bounds__((RMAX * kPairs + 31) / 32 * 32, MB) pair_kerne
         }
         return jq < c.n_jobs;
     };
+    auto a0_of = [&](int64_t b) { return b * c.A_blk; };
     auto e_of = [&](unsigned b) { return (int64_t)b * (Op::kSenseReduce ? 2 * c.E_blk : c.E_blk); };
-    bool have = split_job();
-    if (have) pair_fetch<HM>(op, c, P, Q, ab * c.A_blk, e_of(eb), In);
-    cp_async_commit();
-    if constexpr (Op::kSenseReduce) {
-        if (in2)
-            for (int o = k1; o < c.Lout; o += P) acc[o * kPairs + cp] = make_float2(0.f, 0.f);
-    }
-    cp_async_wait_all();
-    __syncthreads();
-    while (have) {
-        const int64_t a0 = ab * c.A_blk, e0 = e_of(eb);
-        bool last_of_row = true;
-        if (Op::kSenseReduce && eb + 1 < c.n_eb) {
-            ++eb;
-            last_of_row = false;
-        } else {
-            jq += gridDim.x;
-            have = split_job();
-        }
-        // the kernel columns / factor rows of this job, copied under step 1
-        int64_t kc0 = 0;
+    // the kernel columns / factor rows of a job: with its samples for the first job, later ones under step 1
+    int64_t kc0 = 0;
+    auto fetch_side = [&](int64_t a0, int64_t e0) {
         if constexpr (Op::kFusedK) {
-            kc0 = op.kcol(e0);
             if (c.n_k) {
+                kc0 = op.kcol(e0);
                 const int nk = (int)(op.kcol(min(e0 + c.E_blk, c.E) - 1) - kc0) + 1;
                 const float2* src = op.kptr(kc0);  // the columns follow one another
                 for (int i = tid; i < nk * L; i += blockDim.x) cp_async8(Ks + i, src + i);
@@ -633,23 +642,48 @@ __global__ void __launch_bounds__((RMAX * kPairs + 31) / 32 * 32, MB) pair_kerne
                 for (int o = tid & 31; o < c.Lout; o += 32) cp_async8(Ss + col * c.s_stride + o, src + o);
             }
         }
+    };
+    bool have = split_job(), first = true;
+    if (have) {
+        pair_fetch<HM>(op, c, a0_of(ab), e_of(eb), In, Rs);
+        fetch_side(a0_of(ab), e_of(eb));
+    }
+    cp_async_commit();
+    if constexpr (Op::kSenseReduce) {
+        if (in2)
+            for (int o = k1; o < c.Lout; o += P) acc[o * kPairs + cp] = make_float2(0.f, 0.f);
+    }
+    cp_async_wait_all();
+    __syncthreads();
+    while (have) {
+        const int64_t a0 = a0_of(ab), e0 = e_of(eb);
+        bool last_of_row = true;
+        if (Op::kSenseReduce && eb + 1 < c.n_eb) {
+            ++eb;
+            last_of_row = false;
+        } else {
+            jq += gridDim.x;
+            have = split_job();
+        }
+        if (!first) fetch_side(a0, e0);
+        first = false;
         if (in1) {
             const PairCols k = pair_cols<Op>(c, a0, e0, cp);
             radix_switch<RMIN, RMAX, PT>(P, [&](auto rc) {
-                pair_step1<decltype(rc)::value, Op, HM, INV>(op, c, L, Q, k, t, cp, tw, In, Y);
+                pair_step1<decltype(rc)::value, Op, HM, INV>(op, c, L, Q, k, t, cp, tw, In, Rs, a0, Y);
             });
         }
         if (Op::kFusedK || Op::kSenseReduce) cp_async_wait_all();
         __syncthreads();
-        if (!INPL && have) pair_fetch<HM>(op, c, P, Q, ab * c.A_blk, e_of(eb), In);
+        if (!INPL && have) pair_fetch<HM>(op, c, a0_of(ab), e_of(eb), In, Rs);
         const PairCols k = pair_cols<Op>(c, a0, e0, cp2);
         radix_switch<RMIN, RMAX, QT>(Q, [&](auto rc) {
             constexpr int R = decltype(rc)::value;
             c2 u[R];
             if (in2) pair_read2<R, Op, INV>(k1, cp2, Y, u);
-            if constexpr (INPL && PT != 0) {
+            if constexpr (INPL && kEarly) {
                 __syncthreads();
-                if (have) pair_fetch<HM>(op, c, P, Q, ab * c.A_blk, e_of(eb), In);
+                if (have) pair_fetch<HM>(op, c, a0_of(ab), e_of(eb), In, Rs);
             }
             if (in2) {
                 if constexpr (Op::kFusedK) {
@@ -665,7 +699,8 @@ __global__ void __launch_bounds__((RMAX * kPairs + 31) / 32 * 32, MB) pair_kerne
                         acc[o * kPairs + cp] = r;
                     });
                 } else {
-                    pair_outputs<R, HM>(c, P, k1, [&](int k2, int o) { pair_store(op, c, k, o, u[k2]); });
+                    const PairOut<Op> put(op, c, k);
+                    pair_outputs<R, HM>(c, P, k1, [&](int k2, int o) { put(o, u[k2]); });
                 }
             }
         });
@@ -698,17 +733,18 @@ __global__ void __launch_bounds__((RMAX * kPairs + 31) / 32 * 32, MB) pair_kerne
 #pragma unroll
                     for (int q = 0; q < R; ++q) z[q] = Y[(q * Q + t) * kPairs + cp];
                     c2_dft<R, true>(z);
+                    const PairOut<Op> put(op, c, k3);
 #pragma unroll
                     for (int n1 = 0; n1 < (R + 1) / 2; ++n1) {
                         const int pos = t + Q * n1;
-                        if (R % 2 == 0 || 2 * pos < L) pair_store(op, c, k3, pos, z[n1]);
+                        if (R % 2 == 0 || 2 * pos < L) put(pos, z[n1]);
                     }
                 });
             }
         }
-        if constexpr (INPL && PT == 0) {
+        if constexpr (INPL && !kEarly) {
             __syncthreads();
-            if (have) pair_fetch<HM>(op, c, P, Q, ab * c.A_blk, e_of(eb), In);
+            if (have) pair_fetch<HM>(op, c, a0_of(ab), e_of(eb), In, Rs);
         }
         // the next job's samples are in and nobody reads Y any more
         cp_async_wait_all();
@@ -728,6 +764,10 @@ int launch_pair_inst(const Op& op, PairCfg c, cudaStream_t s, const char* name) 
     c.tw_n = c.ph ? 2 * c.L : c.L;
     size_t smem = (size_t)c.L * kPairs * sizeof(c2) + (size_t)c.tw_n * sizeof(float2);
     if (!INPL) smem += (size_t)c.in_elems * sizeof(float2);
+    if constexpr (Op::kLoadLFast) {
+        c.rows = op.rows_shared(c.E_blk);
+        if (c.rows) smem += (size_t)c.A_blk * c.Lin * sizeof(float2);
+    }
     if (Op::kFusedK) smem += (size_t)c.n_k * c.L * sizeof(float2);
     if (Op::kSenseReduce) smem += (size_t)(c.Lout * kPairs + kCW * c.s_stride) * sizeof(float2);
     const int threads = (std::max(c.P, c.Q) * kPairs + 31) / 32 * 32;
@@ -750,12 +790,10 @@ template <class Op, int HM, bool INV>
 int launch_pair_dir(const Op& op, const PairCfg& c, cudaStream_t s, const char* name) {
     const int r = std::max(c.P, c.Q);
     // the edges of the common matrix sizes have their radices as constants (the run-time switch costs 5 - 15 %)
-    if constexpr ((HM & 3) != 0) {
-        if (c.P == 8 && c.Q == 8) return launch_pair_inst<Op, HM, INV, 8, 8, 8, 8, 8>(op, c, s, name);
-        if (c.P == 8 && c.Q == 16) return launch_pair_inst<Op, HM, INV, 8, 16, 8, 16, 4>(op, c, s, name);
-        if (c.P == 16 && c.Q == 16) return launch_pair_inst<Op, HM, INV, 16, 16, 16, 16, 4>(op, c, s, name);
-        if (c.P == 16 && c.Q == 20) return launch_pair_inst<Op, HM, INV, 16, 20, 16, 20, 3>(op, c, s, name);
-    }
+    if (c.P == 8 && c.Q == 8) return launch_pair_inst<Op, HM, INV, 8, 8, 8, 8, 8>(op, c, s, name);
+    if (c.P == 8 && c.Q == 16) return launch_pair_inst<Op, HM, INV, 8, 16, 8, 16, 4>(op, c, s, name);
+    if (c.P == 16 && c.Q == 16) return launch_pair_inst<Op, HM, INV, 16, 16, 16, 16, 4>(op, c, s, name);
+    if (c.P == 16 && c.Q == 20) return launch_pair_inst<Op, HM, INV, 16, 20, 16, 20, 3>(op, c, s, name);
     if (r <= 16) return launch_pair_inst<Op, HM, INV, 8, 16, 0, 0, 4>(op, c, s, name);
     if (r <= 20) return launch_pair_inst<Op, HM, INV, 9, 20, 0, 0, 3>(op, c, s, name);
     return launch_pair_inst<Op, HM, INV, 10, kRadixMax, 0, 0, 2>(op, c, s, name);

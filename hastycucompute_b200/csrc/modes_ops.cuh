@@ -59,9 +59,15 @@ struct OpModesIn {
         return {d0[i0] * d1[i1]};
     }
     __device__ __forceinline__ float2 cvalue(const CState& st, int l, float2 v) const { return cscale(v, st.sc * d2[l]); }
+    int rows_shared(int) const { return 0; }
+    __device__ __forceinline__ const float2* row(int64_t, int64_t) const { return nullptr; }
+    __device__ __forceinline__ void cstate_row(CState&, const float2*) const {}
     bool vout_even() const { return ((d_a | d_l) & 1) == 0; }
     const void* vout_base() const { return dst; }
-    __device__ __forceinline__ float2* vout(int64_t a, int64_t e) const { return dst + a * d_a + e; }
+    static constexpr bool kVecOut = true;
+    using OState = float2*;
+    __device__ __forceinline__ OState ostate(int64_t a, int64_t e, bool) const { return dst + a * d_a + e; }
+    __device__ __forceinline__ void ostore(OState p, int o, float2 v) const { p[(int64_t)o * d_l] = v; }
     __device__ __forceinline__ int64_t vout_l() const { return d_l; }
     __device__ __forceinline__ c2 vout_value(c2 v) const { return v; }
     __device__ __forceinline__ int64_t kcol(int64_t) const { return 0; }
@@ -100,6 +106,23 @@ struct OpModesOut {
     int64_t rows_f, fstride;  // frames: rows (N0 N1) and mode values (C nm) per frame; rows_f 0: one frame
     __device__ __forceinline__ float2 load(int64_t a, int l, int64_t e) const { return src[a * s_a + (int64_t)l * s_l + e]; }
     static constexpr int kPairShapes = 1;
+    struct OState {
+        float2* p;
+        float sc;
+    };
+    __device__ __forceinline__ OState ostate(int64_t a, int64_t e, bool ok) const {
+        if (!ok) return {f, 0.f};
+        uint32_t al = (uint32_t)a;
+        int64_t fo = 0;
+        if (rows_f) {
+            const uint32_t fr = al / (uint32_t)rows_f;
+            al -= fr * (uint32_t)rows_f;
+            fo = (int64_t)fr * fstride;
+        }
+        const uint32_t i0 = al / (uint32_t)N1, i1 = al - i0 * (uint32_t)N1;
+        return {f + fo + e * nm + (int64_t)al * N2, d0[i0] * d1[i1]};
+    }
+    __device__ __forceinline__ void ostore(const OState& s, int o, float2 v) const { s.p[o] = cscale(v, s.sc * d2[o]); }
     // pair access (fftp.cuh)
     bool vin_even() const { return ((s_a | s_l) & 1) == 0; }
     const void* vin_base() const { return src; }

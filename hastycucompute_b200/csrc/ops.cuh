@@ -30,8 +30,11 @@ struct OpStrided {
     __device__ __forceinline__ int64_t vin_l() const { return s_l; }
     bool vout_even() const { return ((d_a | d_l) & 1) == 0; }
     const void* vout_base() const { return dst; }
-    __device__ __forceinline__ float2* vout(int64_t a, int64_t e) const { return dst + a * d_a + e; }
+    static constexpr bool kVecOut = true;
     __device__ __forceinline__ int64_t vout_l() const { return d_l; }
+    using OState = float2*;
+    __device__ __forceinline__ OState ostate(int64_t a, int64_t e, bool) const { return dst + a * d_a + e; }
+    __device__ __forceinline__ void ostore(OState p, int o, float2 v) const { p[(int64_t)o * d_l] = cscale(v, scale); }
     __device__ __forceinline__ c2 vout_value(c2 v) const { return {f2_mul(v.re, f2_dup(scale)), f2_mul(v.im, f2_dup(scale))}; }
     __device__ __forceinline__ int64_t kcol(int64_t) const { return 0; }
     __device__ __forceinline__ const float2* kptr(int64_t) const { return nullptr; }

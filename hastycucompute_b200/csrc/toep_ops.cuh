@@ -32,15 +32,21 @@ struct OpToepIn {
         if (m2) v = mult_typed(v, m2[idx], in_m2);
         return v;
     }
-    // pair access (fftp.cuh)
-    bool vout_even() const { return ((d_a | d_l) & 1) == 0; }
-    const void* vout_base() const { return dst; }
-    __device__ __forceinline__ float2* vout(int64_t a, int64_t e) const { return dst + a * d_a + e; }
-    __device__ __forceinline__ int64_t vout_l() const { return d_l; }
-    __device__ __forceinline__ c2 vout_value(c2 v) const { return v; }
     struct CState {
         const float2 *f1, *f2;
     };
+    // pair access (fftp.cuh)
+    bool vout_even() const { return ((d_a | d_l) & 1) == 0; }
+    const void* vout_base() const { return dst; }
+    static constexpr bool kVecOut = true;
+    using OState = float2*;
+    __device__ __forceinline__ OState ostate(int64_t a, int64_t e, bool) const { return dst + a * d_a + e; }
+    __device__ __forceinline__ void ostore(OState p, int o, float2 v) const { p[(int64_t)o * d_l] = v; }
+    int rows_shared(int) const { return 0; }
+    __device__ __forceinline__ const float2* row(int64_t, int64_t) const { return nullptr; }
+    __device__ __forceinline__ void cstate_row(CState&, const float2*) const {}
+    __device__ __forceinline__ int64_t vout_l() const { return d_l; }
+    __device__ __forceinline__ c2 vout_value(c2 v) const { return v; }
     __device__ __forceinline__ const float2* cin(int64_t a, int64_t e) const { return in + (cpf ? e % cpf : e) * n + a * N2; }
     __device__ __forceinline__ CState cstate(int64_t a, int64_t e, bool ok) const {
         return {m1 ? m1 + (cpf && ok ? (e / cpf) * n : 0) + a * N2 : nullptr, m2 ? m2 + a * N2 : nullptr};
@@ -77,6 +83,9 @@ struct OpToepInSenseT : OpToepIn {
     __device__ __forceinline__ float2 load(int64_t a, int l, int64_t e) const {
         return cmul(load_col(a, l, e), row_at(a, l, e));
     }
+    // pair access: x is one row for all columns of a CTA within one frame
+    int rows_shared(int eb) const { return cpf == 0 || cpf % eb == 0; }
+    __device__ __forceinline__ void cstate_row(CState& f, const float2* r) const { f.f1 = r; }
     __device__ __forceinline__ float2 cvalue(const CState& f, int l, float2 v) const {
         if constexpr (kDiag) v = cmul(v, f.f2[l]);
         return cmul(v, f.f1[l]);
@@ -135,7 +144,10 @@ struct OpToepMid {
     __device__ __forceinline__ int64_t vin_l() const { return E; }
     bool vout_even() const { return (E & 1) == 0; }
     const void* vout_base() const { return buf; }
-    __device__ __forceinline__ float2* vout(int64_t, int64_t e) const { return buf + e; }
+    static constexpr bool kVecOut = true;
+    using OState = float2*;
+    __device__ __forceinline__ OState ostate(int64_t, int64_t e, bool) const { return buf + e; }
+    __device__ __forceinline__ void ostore(OState p, int o, float2 v) const { p[(int64_t)o * E] = v; }
     __device__ __forceinline__ int64_t vout_l() const { return E; }
     __device__ __forceinline__ c2 vout_value(c2 v) const { return v; }
     int64_t cols_per_kernel() const { return B; }
@@ -178,6 +190,19 @@ struct OpToepOutFlat {
     float2* out;
     int64_t N2, n;
     __device__ __forceinline__ float2 load(int64_t a, int l, int64_t e) const { return src[a * s_a + (int64_t)l * s_l + e]; }
+    struct OState {
+        int64_t idx, eo;  // image index of output 0, offset of the batch
+    };
+    __device__ __forceinline__ OState ostate(int64_t a, int64_t e, bool) const { return {a * N2, e * n}; }
+    __device__ __forceinline__ void ostore(const OState& s, int o, float2 v) const {
+        const int64_t idx = s.idx + o;
+        if (m1) v = mult_typed(v, m1[idx], out_m1);
+        if (m2) v = mult_typed(v, m2[idx], out_m2);
+        if (io_mult) v = mult_typed(v, in[s.eo + idx], io_mult);
+        float2* d = out + s.eo + idx;
+        if (accumulate) v = cadd(v, *d);
+        *d = v;
+    }
     // pair access (fftp.cuh)
     bool vin_even() const { return ((s_a | s_l) & 1) == 0; }
     const void* vin_base() const { return src; }
@@ -235,6 +260,7 @@ struct OpToepOutSense {
     }
     __device__ __forceinline__ float2 load(int64_t a, int l, int64_t e) const { return src[a * s_a + (int64_t)l * s_l + e]; }
     __device__ __forceinline__ const float2* sample_ptr(int64_t a, int l, int64_t e) const { return src + a * s_a + (int64_t)l * s_l + e; }
+    using OState = int;  // (no column outputs)
     // pair access (fftp.cuh)
     bool vin_even() const { return ((s_a | s_l) & 1) == 0; }
     const void* vin_base() const { return src; }
