@@ -11,6 +11,7 @@
 
 #include "nufft.cuh"
 #include "modes_ops.cuh"
+#include "spread_walk.cuh"
 
 namespace hb {
 
@@ -63,6 +64,7 @@ struct FoldArgs {
     const int* foff;  // frame point offsets (nullptr: one frame)
     int nfr;
     int ntf;          // bins per frame
+    int sub;          // sort keys per bin: 8 = the first z cell within the bin, 1 = the bin alone
 };
 
 __device__ __forceinline__ float fold_fine(float x, float scale, int nf) {
@@ -85,7 +87,7 @@ __device__ __forceinline__ int first_cell(float u, float hw, int nf) {
 __global__ void k_fold_bin(const FoldArgs a) {
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= a.M) return;
-    int b[3];
+    int b[3], z = 0;
 #pragma unroll
     for (int ax = 0; ax < 3; ++ax) {
         if (a.c[ax] == nullptr) {
@@ -99,9 +101,12 @@ __global__ void k_fold_bin(const FoldArgs a) {
         }
         const float u = fold_fine(x, a.scale[ax], a.nf[ax]);
         a.u[ax][j] = u;
-        b[ax] = first_cell(u, a.hw, a.nf[ax]) / a.T[ax];
+        const int c = first_cell(u, a.hw, a.nf[ax]);
+        b[ax] = c / a.T[ax];
+        if (ax == 0) z = c - b[0] * a.T[0];
     }
-    const int bin = (b[0] * a.nb[1] + b[1]) * a.nb[2] + b[2] + frame_of_point(a.foff, a.nfr, j) * a.ntf;
+    int bin = (b[0] * a.nb[1] + b[1]) * a.nb[2] + b[2] + frame_of_point(a.foff, a.nfr, j) * a.ntf;
+    if (a.sub > 1) bin = bin * a.sub + z;
     a.binid[j] = bin;
     a.rank[j] = atomicAdd(&a.count[bin], 1);
 }
@@ -286,6 +291,37 @@ __global__ void k_tile_parts_fill(const int* cnt, const int* off, int64_t ntiles
     if (tile >= ntiles) return;
     const int n = cnt[tile], o = off[tile];
     for (int q = 0; q < n; ++q) parts[o + q] = make_int4((int)tile, q, n, o);
+}
+
+// Segments of the walking kernel: cnt[seg] = parts of a segment with more than maxp candidates (0 otherwise),
+// pcnt[seg] = the scratch planes they need (every part stores its first cells' planes and W more at most).
+__global__ void k_walk_count(const GridGeom g, const WalkArgs w, int W, int maxp, int* cnt, int* pcnt) {
+    const int64_t seg = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (seg >= w.nseg) return;
+    int fr, ts, ty, tx;
+    walk_segment(g, w, seg, fr, ts, ty, tx);
+    const int ncell = walk_planes(g, w, ts) + W - 1;
+    int64_t total = 0;
+    for (int b = 0; b < 4; ++b) {
+        for (int r = 0; r < ncell;) {
+            int z = ts * w.sp - (W - 1) + r;
+            if (z < 0) z += g.nf[0];
+            const int n = min(8 - (z & 7), ncell - r);  // cells of one bin follow one another
+            const int64_t f = walk_bin(g, fr, z, ty, tx, b);
+            total += w.fine[f + n] - w.fine[f];
+            r += n;
+        }
+    }
+    const int k = total > maxp ? (int)((total + maxp - 1) / maxp) : 0;
+    cnt[seg] = k;
+    pcnt[seg] = k ? ncell + k * W : 0;
+}
+
+__global__ void k_walk_fill(const int* cnt, const int* off, const int* poff, int64_t nseg, int4* parts) {
+    const int64_t seg = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (seg >= nseg) return;
+    const int n = cnt[seg], o = off[seg];
+    for (int q = 0; q < n; ++q) parts[o + q] = make_int4((int)seg, q, n, poff[seg]);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1102,12 +1138,19 @@ int plan_make(NufftPlan* p, int type, int dim, const int64_t* nmodes, int sign, 
     }
     // lanes-on-transforms spreading: 8^3 (3-D) or 16x32 (2-D) tiles, widths 4..8, more than four
     // transforms, and at least two tiles along every non-unit axis (so no footprint wraps onto its
-    // own tile)
+    // own tile). 3-D widths 4..7 walk along z, for any number of transforms, in 0.25 - 0.95 of the tile kernels'
+    // time at every size tried (160^3, 32 transforms, 6.1 M points, w = 6: 20.1 -> 12.4 ms; 128^3 x 16, 2 M
+    // points, w = 4: 3.35 -> 2.11; 64^3 x 32, 0.5 M, w = 7: 2.43 -> 2.24; 64^3 x 8, 131 k, w = 4: 0.26 ->
+    // 0.16; 150^3 x 6, 40 k, w = 6: 0.55 -> 0.42; one transform 128^3, 2 M, w = 4: 2.86 -> 0.68; four 64^3,
+    // 0.3 M, w = 5: 0.78 -> 0.33). At w = 8 the walk's 64 registers of cells spill (64^3 x 32, 0.5 M: 2.99 ->
+    // 6.01 ms).
     {
-        bool ok = (dim == 3 || dim == 2) && w >= 4 && w <= 8 && ntransf >= 5;
+        bool ok = (dim == 3 || dim == 2) && w >= 4 && w <= 8;
         for (int ax = 3 - dim; ax < 3; ++ax) ok = ok && g.nb[ax] >= 2;
-        p->lc = p->lc_ok = ok;
-        p->lc_cc = ntransf >= 17 ? 32 : (ntransf >= 9 ? 16 : 8);
+        p->lc = p->lc_ok = ok && ntransf >= 5;
+        p->lc_cc = ntransf >= 17 ? 32 : (ntransf >= 9 ? 16 : (ntransf >= 5 ? 8 : pow2ceil(ntransf)));
+        p->walk = p->walk_ok = ok && dim == 3 && type == 1 && w <= 7;
+        p->sub = p->walk ? 8 : 1;
         p->st_ok = type == 2 && dim == 3 && w >= 4 && w <= 7;
         p->st = false;
     }
@@ -1153,14 +1196,43 @@ int plan_make(NufftPlan* p, int type, int dim, const int64_t* nmodes, int sign, 
 // of up to 2^d tiles; aim at about 32 subproblems per SM so that the dense tiles of centre-heavy
 // trajectories (radial, spirals) split across the GPU, with at least 256 and at most 4096
 // candidates (large problems keep long chunks per CTA).
-static int auto_subproblem(int64_t M, const GridGeom& g) {
-    int64_t cand = M;
-    for (int ax = 0; ax < 3; ++ax)
+static int auto_subproblem(int64_t M, const GridGeom& g, int tiles_per_point = 0) {
+    int64_t cand = M * (tiles_per_point ? tiles_per_point : 1);
+    for (int ax = 0; ax < 3 && !tiles_per_point; ++ax)
         if (g.nb[ax] > 1) cand *= 2;
     const int64_t want = cand / ((int64_t)kNumSMs * 32);
     int m = 256;
     while (m < want && m < 4096) m <<= 1;
     return m;
+}
+
+// Segment length of the walking kernel: up to four tiles (a candidate within W - 1 cells below a segment is
+// visited by both: 1.16 visits per point at 32 planes and W = 6, 1.6 at 8), fewer where that leaves less than
+// three segments per resident CTA; a segment and its W - 1 cells below must not wrap onto themselves. Returns the
+// number of segments.
+static int64_t walk_segments(NufftPlan* p) {
+    const GridGeom& g = p->g;
+    const int64_t slots = (int64_t)kNumSMs * (p->lc_cc == 32 ? 1 : p->lc_cc == 16 ? 2 : p->lc_cc == 8 ? 3 : 8);
+    const int64_t cols = (int64_t)g.nb[1] * g.nb[2] * g.nfr * ceil_div(g.C, p->lc_cc);
+    int t = std::min(4, g.nb[0] - 1);
+    while (t > 1 && cols * ceil_div(g.nb[0], t) < 3 * slots) --t;
+    p->walk_sp = 8 * t;
+    p->walk_ns = (int)ceil_div(g.nb[0], t);
+    return (int64_t)p->walk_ns * g.nb[1] * g.nb[2] * g.nfr;
+}
+
+static WalkArgs walk_args(const NufftPlan* p) {
+    WalkArgs w{};
+    w.sp = p->walk_sp;
+    w.ns = p->walk_ns;
+    w.nseg = (int64_t)p->walk_ns * p->g.nb[1] * p->g.nb[2] * p->g.nfr;
+    w.fine = p->bin_start;
+    w.parts = p->dense_parts;
+    w.n_parts = (int)p->n_parts;
+    w.range = p->walk_range;
+    w.scratch = p->dense_scratch;
+    w.err = p->d_err;
+    return w;
 }
 
 // Job list of the staged interpolation kernel for the current points (type-2 plans).
@@ -1198,7 +1270,7 @@ int plan_setpts_frames(NufftPlan* p, int nframes, const int64_t* npts, const flo
         HB_REQUIRE(M < (int64_t)0x7fffffff, HB_ERR_INVALID_ARG, "M must be in [0, 2^31)");
         hoff[(size_t)f + 1] = (int)M;
     }
-    HB_REQUIRE((int64_t)p->g.ntf * nframes < (int64_t)0x7fffffff, HB_ERR_INVALID_ARG, "too many frames for the grid");
+    HB_REQUIRE((int64_t)p->g.ntf * nframes * p->sub < (int64_t)0x7fffffff, HB_ERR_INVALID_ARG, "too many frames for the grid");
     HB_REQUIRE(p->g.Nm[0] * p->g.Nm[1] * nframes < ((int64_t)1 << 32), HB_ERR_INVALID_ARG, "too many frames for the modes");
     // grids and per-bin scratch for nframes frames (grown, never shrunk)
     if (nframes > p->frames_cap) {
@@ -1211,7 +1283,7 @@ int plan_setpts_frames(NufftPlan* p, int nframes, const int64_t* npts, const flo
         HB_TRY(dev_alloc(p, (void**)&p->Y, sizeof(float2) * p->Y_elems * nframes, "pass buffer (frames)"));
         p->frames_cap = nframes;
     }
-    const int64_t nbins_all = p->g.ntf * nframes;
+    const int64_t nbins_all = p->g.ntf * nframes * p->sub;  // sort keys
     if (nbins_all > p->nbins_cap) {
         for (int** q : {&p->bin_start, &p->tmp_count, &p->tmp_ecnt, &p->tmp_eoff, &p->tmp_sums}) {
             if (*q) cudaFree(*q);
@@ -1231,7 +1303,8 @@ int plan_setpts_frames(NufftPlan* p, int nframes, const int64_t* npts, const flo
     }
     if (nframes > 1) HB_CUDA(cudaMemcpyAsync(p->foff, hoff.data(), sizeof(int) * (nframes + 1), cudaMemcpyHostToDevice, s));
     g.nfr = nframes;
-    p->nbins = nbins_all;
+    p->nbins = p->g.ntf * nframes;
+    const int64_t nkeys = nbins_all;
     const float* cu[3] = {c0, c1, c2};
     const float* ca[3] = {nullptr, nullptr, nullptr};
     for (int i = 0; i < g.dim; ++i) {
@@ -1284,7 +1357,7 @@ int plan_setpts_frames(NufftPlan* p, int nframes, const int64_t* npts, const flo
     int *binid = p->tmp_binid, *rank = p->tmp_rank, *count = p->tmp_count, *ecnt = p->tmp_ecnt, *eoff = p->tmp_eoff;
     do {
         cudaError_t e = cudaSuccess;
-        if ((e = cudaMemsetAsync(count, 0, sizeof(int) * (p->nbins + 1), s)) != cudaSuccess ||
+        if ((e = cudaMemsetAsync(count, 0, sizeof(int) * (nkeys + 1), s)) != cudaSuccess ||
             (e = cudaMemsetAsync(p->d_err, 0, sizeof(int), s)) != cudaSuccess) {
             set_error(std::string("setpts memset: ") + cudaGetErrorString(e));
             st = HB_ERR_CUDA;
@@ -1309,10 +1382,11 @@ int plan_setpts_frames(NufftPlan* p, int nframes, const int64_t* npts, const flo
             fa.foff = nframes > 1 ? p->foff : nullptr;
             fa.nfr = nframes;
             fa.ntf = (int)g.ntf;
+            fa.sub = p->sub;
             k_fold_bin<<<(unsigned)ceil_div(M, 256), 256, 0, s>>>(fa);
             if ((st = check_launch("k_fold_bin")) != HB_OK) break;
         }
-        if ((st = exclusive_scan_int(count, p->bin_start, p->nbins, s, p->tmp_sums)) != HB_OK) break;
+        if ((st = exclusive_scan_int(count, p->bin_start, nkeys, s, p->tmp_sums)) != HB_OK) break;
         if (M > 0) {
             k_scatter_sorted<<<(unsigned)ceil_div(M, 256), 256, 0, s>>>(u[0], u[1], u[2], binid, rank, p->bin_start,
                                                                        ca[0] ? p->su[0] : nullptr, ca[1] ? p->su[1] : nullptr,
@@ -1322,7 +1396,54 @@ int plan_setpts_frames(NufftPlan* p, int nframes, const int64_t* npts, const flo
         // unit axes: sorted coordinate arrays hold zeros
         for (int ax = 0; ax < 3; ++ax)
             if (!ca[ax] && p->su[ax] && M > 0) cudaMemsetAsync(p->su[ax], 0, sizeof(float) * M, s);
-        if (p->type == 1 && p->lc) {
+        if (p->type == 1 && p->walk) {
+            if (p->maxp_auto) p->maxp = std::max(512, auto_subproblem(M, g, 4));
+            const int64_t nseg = walk_segments(p);
+            const WalkArgs wa = walk_args(p);
+            // the bin counts are done with: scratch for the planes per segment and their offsets
+            int *pcnt = count, *poff = count + nseg + 1;
+            const int W = g.wa[2];
+            k_walk_count<<<(unsigned)ceil_div(nseg, 128), 128, 0, s>>>(g, wa, W, p->maxp, ecnt, pcnt);
+            if ((st = check_launch("k_walk_count")) != HB_OK) break;
+            if ((st = exclusive_scan_int(ecnt, eoff, nseg, s, p->tmp_sums)) != HB_OK) break;
+            if ((st = exclusive_scan_int(pcnt, poff, nseg, s, p->tmp_sums)) != HB_OK) break;
+            int n_parts = 0, n_planes = 0;
+            if ((e = cudaMemcpyAsync(&n_parts, eoff + nseg, sizeof(int), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
+                (e = cudaMemcpyAsync(&n_planes, poff + nseg, sizeof(int), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
+                (e = cudaStreamSynchronize(s)) != cudaSuccess) {
+                set_error(std::string("setpts sync: ") + cudaGetErrorString(e));
+                st = HB_ERR_CUDA;
+                break;
+            }
+            if (n_parts > p->parts_cap) {
+                if (p->dense_parts) cudaFree(p->dense_parts);
+                p->dense_parts = nullptr;
+                p->parts_cap = 0;
+                if ((st = dev_alloc(p, (void**)&p->dense_parts, sizeof(int4) * n_parts, "dense segment parts")) != HB_OK) break;
+                p->parts_cap = n_parts;
+            }
+            if (n_parts > p->walk_range_cap) {
+                if (p->walk_range) cudaFree(p->walk_range);
+                p->walk_range = nullptr;
+                p->walk_range_cap = 0;
+                if ((st = dev_alloc(p, (void**)&p->walk_range, sizeof(int2) * n_parts, "dense segment ranges")) != HB_OK) break;
+                p->walk_range_cap = n_parts;
+            }
+            const size_t need = sizeof(float2) * (size_t)n_planes * 64 * g.C;
+            if (need > p->scratch_cap) {
+                if (p->dense_scratch) cudaFree(p->dense_scratch);
+                p->dense_scratch = nullptr;
+                p->scratch_cap = 0;
+                if ((st = dev_alloc(p, (void**)&p->dense_scratch, need, "dense segment planes")) != HB_OK) break;
+                p->scratch_cap = need;
+            }
+            p->n_parts = n_parts;
+            if (n_parts > 0) {
+                k_walk_fill<<<(unsigned)ceil_div(nseg, 256), 256, 0, s>>>(ecnt, eoff, poff, nseg, p->dense_parts);
+                if ((st = check_launch("k_walk_fill")) != HB_OK) break;
+            }
+            p->n_extra = 0;
+        } else if (p->type == 1 && p->lc) {
             if (p->maxp_auto) p->maxp = auto_subproblem(M, g);
             TileNbr tn;
             for (int ax = 0; ax < 3; ++ax) tn.nb[ax] = g.nb[ax];
@@ -1583,7 +1704,17 @@ int plan_execute(NufftPlan* p, const float2* in, float2* out, cudaStream_t s) {
             HB_TRY(check_launch("k_interleave_in"));
         }
         GridArgs a = grid_args(p);
-        if (p->lc)
+        if (p->walk) {
+            const WalkArgs w = walk_args(p);
+            switch (p->lc_cc) {
+                case 1: HB_TRY(spread_walk_cc1(p, a, w, s)); break;
+                case 2: HB_TRY(spread_walk_cc2(p, a, w, s)); break;
+                case 4: HB_TRY(spread_walk_cc4(p, a, w, s)); break;
+                case 8: HB_TRY(spread_walk_cc8(p, a, w, s)); break;
+                case 16: HB_TRY(spread_walk_cc16(p, a, w, s)); break;
+                default: HB_TRY(spread_walk_cc32(p, a, w, s)); break;
+            }
+        } else if (p->lc)
             HB_TRY(p->lc_cc == 8 ? spread_lc_cc8(p, a, s) : (p->lc_cc == 16 ? spread_lc_cc16(p, a, s) : spread_lc_cc32(p, a, s)));
         else
             HB_TRY(dispatch_cc(spread_cc(g), p, a, s, true));
@@ -1682,7 +1813,9 @@ int plan_set_spread_kernel(NufftPlan* p, int kind, int transforms_per_cta) {
     HB_REQUIRE(transforms_per_cta == 0 || transforms_per_cta == 8 || transforms_per_cta == 16 || transforms_per_cta == 32,
                HB_ERR_INVALID_ARG, "transforms per CTA must be 0 (automatic), 8, 16 or 32");
     p->lc = base == HB_SPREAD_CELLS ? false : p->lc_ok;
-    if (transforms_per_cta) p->lc_cc = transforms_per_cta;
+    p->walk = base == HB_SPREAD_CELLS ? false : p->walk_ok;
+    p->sub = p->walk ? 8 : 1;
+    if (transforms_per_cta && p->lc_ok) p->lc_cc = transforms_per_cta;
     return HB_OK;
 }
 
@@ -1757,6 +1890,9 @@ void plan_free(NufftPlan* p) {
     if (p->st_jobs) cudaFree(p->st_jobs);
     p->st_jobs = nullptr;
     p->n_st_jobs = p->st_cap = 0;
+    if (p->walk_range) cudaFree(p->walk_range);
+    p->walk_range = nullptr;
+    p->walk_range_cap = 0;
     p->dense_parts = nullptr;
     p->dense_scratch = nullptr;
     p->parts_cap = 0;

@@ -93,6 +93,14 @@ struct NufftPlan {
     bool lc = false;
     bool lc_ok = false;
     int lc_cc = 0;
+    // walking spreading (k_spread_walk, 3-D): usable (walk_ok), chosen (walk), its transforms per CTA (lc_cc). Its points are sorted by (bin, z cell), `sub` keys per bin; segments of walk_sp planes,
+    // walk_ns per column; first and last cell of every part
+    bool walk = false;
+    bool walk_ok = false;
+    int sub = 1;
+    int walk_sp = 8, walk_ns = 1;
+    int2* walk_range = nullptr;
+    int64_t walk_range_cap = 0;
     int interp_cc = 0;  // interpolation: transforms per lane group (0 = the spreading rule)
     int4* dense_parts = nullptr;
     int64_t n_parts = 0, parts_cap = 0;
@@ -153,6 +161,15 @@ __device__ __forceinline__ int split_frame_tile(const GridGeom& g, int& tile) {
 int spread_lc_cc8(const NufftPlan* p, const GridArgs& a, cudaStream_t s);
 int spread_lc_cc16(const NufftPlan* p, const GridArgs& a, cudaStream_t s);
 int spread_lc_cc32(const NufftPlan* p, const GridArgs& a, cudaStream_t s);
+
+// Walking spreading (spread_walk.cuh; instances in spread_walk{1,2,4,8,16,32}.cu) for plans with p->walk set.
+struct WalkArgs;
+int spread_walk_cc1(const NufftPlan* p, const GridArgs& a, const WalkArgs& w, cudaStream_t s);
+int spread_walk_cc2(const NufftPlan* p, const GridArgs& a, const WalkArgs& w, cudaStream_t s);
+int spread_walk_cc4(const NufftPlan* p, const GridArgs& a, const WalkArgs& w, cudaStream_t s);
+int spread_walk_cc8(const NufftPlan* p, const GridArgs& a, const WalkArgs& w, cudaStream_t s);
+int spread_walk_cc16(const NufftPlan* p, const GridArgs& a, const WalkArgs& w, cudaStream_t s);
+int spread_walk_cc32(const NufftPlan* p, const GridArgs& a, const WalkArgs& w, cudaStream_t s);
 
 int plan_make(NufftPlan* p, int type, int dim, const int64_t* nmodes, int sign, int ntransf, float tol,
               int width, double upsampfac, int method);

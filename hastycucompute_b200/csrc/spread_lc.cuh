@@ -1,4 +1,5 @@
-// Type-1 spreading with the transforms on the lanes.
+// Type-1 spreading with the transforms on the lanes: 2-D plans, and 3-D plans of width 8 (widths 4 .. 7 walk
+// along z, spread_walk.cuh).
 //
 // One CTA owns one tile of the fine grid (8x8x8 in 3-D, 16x32 in 2-D) for CC transforms. The 32
 // lanes of a warp are G = 32/CC groups of CC transforms; every thread keeps 4 rows x 8 cells of
@@ -422,12 +423,16 @@ inline int launch_spread_lc(const NufftPlan* p, const GridArgs& a, cudaStream_t 
 
 template <int CC, bool D3>
 inline int launch_spread_lc_w(const NufftPlan* p, const GridArgs& a, cudaStream_t s) {
-    switch (p->g.wa[2]) {
-        case 4: return launch_spread_lc<CC, 4, D3>(p, a, s);
-        case 5: return launch_spread_lc<CC, 5, D3>(p, a, s);
-        case 6: return launch_spread_lc<CC, 6, D3>(p, a, s);
-        case 7: return launch_spread_lc<CC, 7, D3>(p, a, s);
-        default: return launch_spread_lc<CC, 8, D3>(p, a, s);
+    if constexpr (D3) {
+        return launch_spread_lc<CC, 8, true>(p, a, s);
+    } else {
+        switch (p->g.wa[2]) {
+            case 4: return launch_spread_lc<CC, 4, false>(p, a, s);
+            case 5: return launch_spread_lc<CC, 5, false>(p, a, s);
+            case 6: return launch_spread_lc<CC, 6, false>(p, a, s);
+            case 7: return launch_spread_lc<CC, 7, false>(p, a, s);
+            default: return launch_spread_lc<CC, 8, false>(p, a, s);
+        }
     }
 }
 
