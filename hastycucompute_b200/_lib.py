@@ -43,6 +43,8 @@ SIGNATURES = {
     "hb_nufft_get_info": (_i, [_vp, _pi64, C.POINTER(_i), C.POINTER(_d), C.POINTER(_sz)]),
     "hb_toeplitz_kernel": (_i, [_i, _pi64, _i64, _vp, _vp, _vp, _vp, _vp, _i, _vp]),
     "hb_toeplitz_kernels_frames": (_i, [_i, _pi64, _i, _pi64, _vp, _vp, _vp, _vp, _vp, _i, _vp]),
+    "hb_toeplitz_kernels_workspace_size": (_i, [_i, _pi64, _i, _pi64, _i, C.POINTER(_sz)]),
+    "hb_toeplitz_kernels_frames_ws": (_i, [_i, _pi64, _i, _pi64, _vp, _vp, _vp, _vp, _vp, _i, _vp, _sz, _vp]),
     "hb_transform_toeplitz_kernel": (_i, [_i, _pi64, _vp, _vp, _vp]),
     "hb_toeplitz_workspace_size": (_i, [_i, _pi64, _i64, C.POINTER(_sz)]),
     "hb_toeplitz_multiplication": (_i, [_i, _pi64, _i64, _vp, _vp, _vp, _vp, _sz, _vp, _vp,

@@ -16,7 +16,8 @@ const char* get_error() { return g_last_error.c_str(); }
 int toeplitz_kernel(int dim, const int64_t* kshape, int64_t M, const float* c0, const float* c1, const float* c2,
                     const void* nudata, void* kout, int width, cudaStream_t s);
 int toeplitz_kernel_frames(int dim, const int64_t* kshape, int nframes, const int64_t* npts, const float* c0,
-                           const float* c1, const float* c2, const void* nudata, void* kout, int width, cudaStream_t s);
+                           const float* c1, const float* c2, const void* nudata, void* kout, int width, void* workspace, size_t workspace_bytes, cudaStream_t s);
+int toeplitz_kernel_workspace(int dim, const int64_t* kshape, int nframes, const int64_t* npts, int width, size_t* bytes);
 int transform_toeplitz_kernel(int dim, const int64_t* kshape, const void* kin, void* kout, cudaStream_t s);
 int toeplitz_workspace_size(int dim, const int64_t* shape, int64_t nbatch, size_t* bytes);
 int toeplitz_multiplication(int dim, const int64_t* shape, int64_t nbatch, const void* input, void* output,
@@ -220,7 +221,22 @@ int hb_toeplitz_kernels_frames(int dim, const int64_t* kernel_shape, int nframes
                                void* kernel_out, int kernel_width, void* stream) {
     HB_GUARD({
         return hb::toeplitz_kernel_frames(dim, kernel_shape, nframes, npts, coord0, coord1, coord2, nudata, kernel_out,
-                                          kernel_width, as_stream(stream));
+                                          kernel_width, nullptr, 0, as_stream(stream));
+    })
+}
+
+int hb_toeplitz_kernels_workspace_size(int dim, const int64_t* kernel_shape, int nframes, const int64_t* npts,
+                                       int kernel_width, size_t* bytes) {
+    HB_GUARD({ return hb::toeplitz_kernel_workspace(dim, kernel_shape, nframes, npts, kernel_width, bytes); })
+}
+
+int hb_toeplitz_kernels_frames_ws(int dim, const int64_t* kernel_shape, int nframes, const int64_t* npts,
+                                  const float* coord0, const float* coord1, const float* coord2, const void* nudata,
+                                  void* kernel_out, int kernel_width, void* workspace, size_t workspace_bytes,
+                                  void* stream) {
+    HB_GUARD({
+        return hb::toeplitz_kernel_frames(dim, kernel_shape, nframes, npts, coord0, coord1, coord2, nudata, kernel_out,
+                                          kernel_width, workspace, workspace_bytes, as_stream(stream));
     })
 }
 

@@ -1065,7 +1065,15 @@ __global__ void __launch_bounds__(kGridThreads) k_interp_grad(const GridArgs a, 
 // ---------------------------------------------------------------------------------------------
 // plan lifecycle
 
+// Device memory of a plan: from its arena (a caller's workspace, 256-byte pieces, never freed one by one)
+// while that lasts, else cudaMalloc.
 static int dev_alloc(NufftPlan* p, void** ptr, size_t bytes, const char* what) {
+    const size_t piece = arena_piece(bytes);
+    if (p->arena && p->arena_used + piece <= p->arena_bytes) {
+        *ptr = p->arena + p->arena_used;
+        p->arena_used += piece;
+        return HB_OK;
+    }
     cudaError_t e = cudaMalloc(ptr, bytes ? bytes : 16);
     if (e != cudaSuccess) {
         *ptr = nullptr;
@@ -1076,6 +1084,27 @@ static int dev_alloc(NufftPlan* p, void** ptr, size_t bytes, const char* what) {
     p->device_bytes += bytes;
     return HB_OK;
 }
+
+static void dev_free(NufftPlan* p, void* ptr) {
+    if (!ptr) return;
+    if (p->arena && (char*)ptr >= p->arena && (char*)ptr < p->arena + p->arena_bytes) return;
+    cudaFree(ptr);
+}
+
+// tiles: 8^3 (3-D), 16x32 (2-D), 256 (1-D); wider kernels need tiles >= w-1
+static int tile_edge(int dim, int ax, int w) {
+    if (dim == 3) return w <= 9 ? 8 : 16;
+    if (dim == 2) return ax == 1 ? 16 : 32;
+    return 256;
+}
+
+int64_t plan_fine_size(int64_t N, int dim, int ax, int width) {
+    const int w = width > 0 ? std::min(width, kMaxWidth) : 6;
+    return fine_size(N, 2.0, w, tile_edge(dim, ax, w));
+}
+
+int plan_alloc(NufftPlan* p, void** ptr, size_t bytes, const char* what) { return dev_alloc(p, ptr, bytes, what); }
+void plan_release(NufftPlan* p, void* ptr) { dev_free(p, ptr); }
 
 int plan_make(NufftPlan* p, int type, int dim, const int64_t* nmodes, int sign, int ntransf, float tol, int width,
               double upsampfac, int method) {
@@ -1110,22 +1139,9 @@ int plan_make(NufftPlan* p, int type, int dim, const int64_t* nmodes, int sign, 
         HB_REQUIRE(nmodes[i] >= 1 && nmodes[i] <= (1 << 20), HB_ERR_INVALID_ARG, "nmodes out of range");
         g.Nm[3 - dim + i] = nmodes[i];
     }
-    // tiles: 8^3 (3-D), 16x32 (2-D), 256 (1-D); wider kernels need tiles >= w-1
-    int Tt[3];
-    if (dim == 3) {
-        const int e = (w <= 9) ? 8 : 16;
-        Tt[0] = Tt[1] = Tt[2] = e;
-    } else if (dim == 2) {
-        Tt[0] = 1;
-        Tt[1] = 16;
-        Tt[2] = 32;
-    } else {
-        Tt[0] = Tt[1] = 1;
-        Tt[2] = 256;
-    }
     for (int ax = 0; ax < 3; ++ax) {
         const bool unit = (ax < 3 - dim);
-        g.T[ax] = unit ? 1 : Tt[ax];
+        g.T[ax] = unit ? 1 : tile_edge(dim, ax, w);
         g.wa[ax] = unit ? 1 : w;
         g.nf[ax] = unit ? 1 : fine_size(g.Nm[ax], p->sigma, w, g.T[ax]);
         g.nb[ax] = g.nf[ax] / g.T[ax];
@@ -1166,7 +1182,8 @@ int plan_make(NufftPlan* p, int type, int dim, const int64_t* nmodes, int sign, 
 
     // FFT plans and deapodisation factors per axis
     for (int ax = 0; ax < 3; ++ax) {
-        if (g.nf[ax] > 1) HB_TRY(fftlen_make(&p->fl[ax], g.nf[ax]));
+        // (a plan in a caller's workspace borrows the thread's tables)
+        if (g.nf[ax] > 1) HB_TRY(p->arena ? cached_len(g.nf[ax], &p->fl[ax]) : fftlen_make(&p->fl[ax], g.nf[ax]));
         std::vector<float> dv((size_t)g.Nm[ax], 1.0f);
         if (g.nf[ax] > 1) {
             const int64_t half = g.Nm[ax] / 2;
@@ -1176,18 +1193,25 @@ int plan_make(NufftPlan* p, int type, int dim, const int64_t* nmodes, int sign, 
             }
         }
         HB_TRY(dev_alloc(p, (void**)&p->deapod[ax], sizeof(float) * dv.size(), "deapod"));
-        HB_CUDA(cudaMemcpy(p->deapod[ax], dv.data(), sizeof(float) * dv.size(), cudaMemcpyHostToDevice));
+        // workspace memory is stream-ordered: earlier work on the stream may still use it
+        if (p->arena)
+            HB_CUDA(cudaMemcpyAsync(p->deapod[ax], dv.data(), sizeof(float) * dv.size(), cudaMemcpyHostToDevice, p->arena_stream));
+        else
+            HB_CUDA(cudaMemcpy(p->deapod[ax], dv.data(), sizeof(float) * dv.size(), cudaMemcpyHostToDevice));
     }
     p->X_elems = (size_t)g.nf[0] * g.nf[1] * g.nf[2] * g.C;
     HB_REQUIRE(p->X_elems < ((size_t)1 << 32), HB_ERR_INVALID_ARG,
                "fine grid x ntransf must hold fewer than 2^32 values; split the transforms");
     p->Y_elems = (size_t)g.Nm[0] * g.nf[1] * g.nf[2] * g.C;
     g.fgrid = (int64_t)p->X_elems;
-    p->frames_cap = 1;
-    HB_TRY(dev_alloc(p, (void**)&p->X, sizeof(float2) * p->X_elems, "fine grid"));
-    HB_TRY(dev_alloc(p, (void**)&p->Y, sizeof(float2) * p->Y_elems, "pass buffer"));
-    HB_TRY(dev_alloc(p, (void**)&p->bin_start, sizeof(int) * (p->nbins + 1), "bins"));
-    p->nbins_cap = p->nbins;
+    p->frames_cap = 0;
+    if (!p->arena) {  // (in a workspace the first setpts places the grids, once, for all its frames)
+        HB_TRY(dev_alloc(p, (void**)&p->X, sizeof(float2) * p->X_elems, "fine grid"));
+        HB_TRY(dev_alloc(p, (void**)&p->Y, sizeof(float2) * p->Y_elems, "pass buffer"));
+        p->frames_cap = 1;
+    }
+    p->nbins_cap = p->nbins * p->sub;
+    HB_TRY(dev_alloc(p, (void**)&p->bin_start, sizeof(int) * (p->nbins_cap + 1), "bins"));
     HB_TRY(dev_alloc(p, (void**)&p->d_err, sizeof(int), "error flag"));
     return HB_OK;
 }
@@ -1240,7 +1264,7 @@ static int st_build_jobs(NufftPlan* p, cudaStream_t s) {
     int n_jobs = 0;
     HB_TRY(interp_st_jobs(p->bin_start, p->nbins, p->g.wa[2], p->tmp_ecnt, p->tmp_eoff, p->tmp_sums, nullptr, &n_jobs, 0, s));
     if (n_jobs > p->st_cap) {
-        if (p->st_jobs) cudaFree(p->st_jobs);
+        dev_free(p, p->st_jobs);
         p->st_jobs = nullptr;
         p->st_cap = 0;
         HB_TRY(dev_alloc(p, (void**)&p->st_jobs, sizeof(int4) * n_jobs, "staged interpolation jobs"));
@@ -1274,8 +1298,8 @@ int plan_setpts_frames(NufftPlan* p, int nframes, const int64_t* npts, const flo
     HB_REQUIRE(p->g.Nm[0] * p->g.Nm[1] * nframes < ((int64_t)1 << 32), HB_ERR_INVALID_ARG, "too many frames for the modes");
     // grids and per-bin scratch for nframes frames (grown, never shrunk)
     if (nframes > p->frames_cap) {
-        if (p->X) cudaFree(p->X);
-        if (p->Y) cudaFree(p->Y);
+        dev_free(p, p->X);
+        dev_free(p, p->Y);
         p->X = p->Y = nullptr;
         p->frames_cap = 0;
         p->pts_set = false;
@@ -1286,7 +1310,7 @@ int plan_setpts_frames(NufftPlan* p, int nframes, const int64_t* npts, const flo
     const int64_t nbins_all = p->g.ntf * nframes * p->sub;  // sort keys
     if (nbins_all > p->nbins_cap) {
         for (int** q : {&p->bin_start, &p->tmp_count, &p->tmp_ecnt, &p->tmp_eoff, &p->tmp_sums}) {
-            if (*q) cudaFree(*q);
+            dev_free(p, *q);
             *q = nullptr;
         }
         p->nbins_cap = 0;
@@ -1295,7 +1319,7 @@ int plan_setpts_frames(NufftPlan* p, int nframes, const int64_t* npts, const flo
         p->nbins_cap = nbins_all;
     }
     if (nframes > 1 && nframes + 1 > p->foff_cap) {
-        if (p->foff) cudaFree(p->foff);
+        dev_free(p, p->foff);
         p->foff = nullptr;
         p->foff_cap = 0;
         HB_TRY(dev_alloc(p, (void**)&p->foff, sizeof(int) * (nframes + 1), "frame offsets"));
@@ -1313,11 +1337,11 @@ int plan_setpts_frames(NufftPlan* p, int nframes, const int64_t* npts, const flo
     }
     if (M > p->M_cap) {
         for (int ax = 0; ax < 3; ++ax) {
-            if (p->su[ax]) cudaFree(p->su[ax]);
+            dev_free(p, p->su[ax]);
             p->su[ax] = nullptr;
         }
-        if (p->perm) cudaFree(p->perm);
-        if (p->inT) cudaFree(p->inT);
+        dev_free(p, p->perm);
+        dev_free(p, p->inT);
         p->perm = nullptr;
         p->inT = nullptr;
         for (int ax = 0; ax < 3; ++ax)
@@ -1340,11 +1364,11 @@ int plan_setpts_frames(NufftPlan* p, int nframes, const int64_t* npts, const flo
     }
     if (M > p->tmp_cap) {
         for (int ax = 0; ax < 3; ++ax) {
-            if (p->tmp_u[ax]) cudaFree(p->tmp_u[ax]);
+            dev_free(p, p->tmp_u[ax]);
             p->tmp_u[ax] = nullptr;
         }
-        if (p->tmp_binid) cudaFree(p->tmp_binid);
-        if (p->tmp_rank) cudaFree(p->tmp_rank);
+        dev_free(p, p->tmp_binid);
+        dev_free(p, p->tmp_rank);
         p->tmp_binid = p->tmp_rank = nullptr;
         p->tmp_cap = 0;
         for (int ax = 0; ax < 3; ++ax)
@@ -1416,14 +1440,14 @@ int plan_setpts_frames(NufftPlan* p, int nframes, const int64_t* npts, const flo
                 break;
             }
             if (n_parts > p->parts_cap) {
-                if (p->dense_parts) cudaFree(p->dense_parts);
+                dev_free(p, p->dense_parts);
                 p->dense_parts = nullptr;
                 p->parts_cap = 0;
                 if ((st = dev_alloc(p, (void**)&p->dense_parts, sizeof(int4) * n_parts, "dense segment parts")) != HB_OK) break;
                 p->parts_cap = n_parts;
             }
             if (n_parts > p->walk_range_cap) {
-                if (p->walk_range) cudaFree(p->walk_range);
+                dev_free(p, p->walk_range);
                 p->walk_range = nullptr;
                 p->walk_range_cap = 0;
                 if ((st = dev_alloc(p, (void**)&p->walk_range, sizeof(int2) * n_parts, "dense segment ranges")) != HB_OK) break;
@@ -1431,7 +1455,7 @@ int plan_setpts_frames(NufftPlan* p, int nframes, const int64_t* npts, const flo
             }
             const size_t need = sizeof(float2) * (size_t)n_planes * 64 * g.C;
             if (need > p->scratch_cap) {
-                if (p->dense_scratch) cudaFree(p->dense_scratch);
+                dev_free(p, p->dense_scratch);
                 p->dense_scratch = nullptr;
                 p->scratch_cap = 0;
                 if ((st = dev_alloc(p, (void**)&p->dense_scratch, need, "dense segment planes")) != HB_OK) break;
@@ -1460,7 +1484,7 @@ int plan_setpts_frames(NufftPlan* p, int nframes, const int64_t* npts, const flo
                 break;
             }
             if (n_parts > p->parts_cap) {
-                if (p->dense_parts) cudaFree(p->dense_parts);
+                dev_free(p, p->dense_parts);
                 p->dense_parts = nullptr;
                 p->parts_cap = 0;
                 if ((st = dev_alloc(p, (void**)&p->dense_parts, sizeof(int4) * n_parts, "dense tile parts")) != HB_OK) break;
@@ -1468,7 +1492,7 @@ int plan_setpts_frames(NufftPlan* p, int nframes, const int64_t* npts, const flo
             }
             const size_t need = sizeof(float2) * (size_t)n_parts * g.T[0] * g.T[1] * g.T[2] * g.C;
             if (need > p->scratch_cap) {
-                if (p->dense_scratch) cudaFree(p->dense_scratch);
+                dev_free(p, p->dense_scratch);
                 p->dense_scratch = nullptr;
                 p->scratch_cap = 0;
                 if ((st = dev_alloc(p, (void**)&p->dense_scratch, need, "dense tile partials")) != HB_OK) break;
@@ -1504,7 +1528,7 @@ int plan_setpts_frames(NufftPlan* p, int nframes, const int64_t* npts, const flo
                 break;
             }
             if (n_extra > p->extra_cap) {
-                if (p->extra) cudaFree(p->extra);
+                dev_free(p, p->extra);
                 p->extra = nullptr;
                 p->extra_cap = 0;
                 if ((st = dev_alloc(p, (void**)&p->extra, sizeof(int4) * n_extra, "spread work list")) != HB_OK) break;
@@ -1512,7 +1536,7 @@ int plan_setpts_frames(NufftPlan* p, int nframes, const int64_t* npts, const flo
             }
             const size_t need = sizeof(float2) * (size_t)n_extra * g.T[0] * g.T[1] * g.T[2] * g.C;
             if (need > p->extra_scratch_cap) {
-                if (p->extra_scratch) cudaFree(p->extra_scratch);
+                dev_free(p, p->extra_scratch);
                 p->extra_scratch = nullptr;
                 p->extra_scratch_cap = 0;
                 if ((st = dev_alloc(p, (void**)&p->extra_scratch, need, "spread partial tiles")) != HB_OK) break;
@@ -1864,33 +1888,33 @@ int plan_coord_grad(NufftPlan* p, const float2* modes, const float2* h, float* g
 
 void plan_free(NufftPlan* p) {
     for (int ax = 0; ax < 3; ++ax) {
-        fftlen_free(&p->fl[ax]);
-        if (p->deapod[ax]) cudaFree(p->deapod[ax]);
-        if (p->su[ax]) cudaFree(p->su[ax]);
+        if (!p->arena) fftlen_free(&p->fl[ax]);
+        dev_free(p, p->deapod[ax]);
+        dev_free(p, p->su[ax]);
         p->deapod[ax] = nullptr;
         p->su[ax] = nullptr;
     }
-    if (p->X) cudaFree(p->X);
-    if (p->Y) cudaFree(p->Y);
-    if (p->foff) cudaFree(p->foff);
+    dev_free(p, p->X);
+    dev_free(p, p->Y);
+    dev_free(p, p->foff);
     p->foff = nullptr;
-    if (p->perm) cudaFree(p->perm);
-    if (p->inT) cudaFree(p->inT);
-    if (p->bin_start) cudaFree(p->bin_start);
-    if (p->extra) cudaFree(p->extra);
-    if (p->extra_scratch) cudaFree(p->extra_scratch);
+    dev_free(p, p->perm);
+    dev_free(p, p->inT);
+    dev_free(p, p->bin_start);
+    dev_free(p, p->extra);
+    dev_free(p, p->extra_scratch);
     p->extra_scratch = nullptr;
-    if (p->d_err) cudaFree(p->d_err);
+    dev_free(p, p->d_err);
     for (int ax = 0; ax < 3; ++ax) {
-        if (p->tmp_u[ax]) cudaFree(p->tmp_u[ax]);
+        dev_free(p, p->tmp_u[ax]);
         p->tmp_u[ax] = nullptr;
     }
-    if (p->dense_parts) cudaFree(p->dense_parts);
-    if (p->dense_scratch) cudaFree(p->dense_scratch);
-    if (p->st_jobs) cudaFree(p->st_jobs);
+    dev_free(p, p->dense_parts);
+    dev_free(p, p->dense_scratch);
+    dev_free(p, p->st_jobs);
     p->st_jobs = nullptr;
     p->n_st_jobs = p->st_cap = 0;
-    if (p->walk_range) cudaFree(p->walk_range);
+    dev_free(p, p->walk_range);
     p->walk_range = nullptr;
     p->walk_range_cap = 0;
     p->dense_parts = nullptr;
@@ -1898,7 +1922,7 @@ void plan_free(NufftPlan* p) {
     p->parts_cap = 0;
     p->scratch_cap = 0;
     for (int** q : {&p->tmp_binid, &p->tmp_rank, &p->tmp_count, &p->tmp_ecnt, &p->tmp_eoff, &p->tmp_sums}) {
-        if (*q) cudaFree(*q);
+        dev_free(p, *q);
         *q = nullptr;
     }
     p->tmp_cap = 0;

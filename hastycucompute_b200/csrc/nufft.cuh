@@ -114,7 +114,14 @@ struct NufftPlan {
     int4* st_jobs = nullptr;
     int64_t n_st_jobs = 0, st_cap = 0;
     size_t device_bytes = 0;
+    // a temporary plan in a caller's workspace (nullptr: the plan owns what it allocates)
+    char* arena = nullptr;
+    size_t arena_bytes = 0, arena_used = 0;
+    cudaStream_t arena_stream = nullptr;
 };
+
+constexpr size_t arena_piece(size_t bytes) { return (bytes + 255) / 256 * 256 + 256; }
+
 
 
 // Arguments of the gridding kernels (spreading and interpolation).
@@ -193,6 +200,13 @@ int interp_st_jobs(const int* bin_start, int64_t ntiles, int w, int* cnt, int* o
                    int64_t jobs_cap, cudaStream_t s);
 int interp_st_run(const NufftPlan* p, const GridArgs& a, cudaStream_t s);
 void plan_free(NufftPlan* p);
+// fine cells along internal axis ax of a type-1 / type-2 plan of N modes there (width <= 0: 6)
+int64_t plan_fine_size(int64_t N, int dim, int ax, int width);
+// memory from the plan's arena or cudaMalloc, and its release
+int plan_alloc(NufftPlan* p, void** ptr, size_t bytes, const char* what);
+void plan_release(NufftPlan* p, void* ptr);
+// the calling thread's twiddle table of length L on the current device (toeplitz.cu)
+int cached_len(int L, FftLen* out);
 
 // Pieces reused by the Toeplitz kernel builder.
 // `sums` (optional): ceil(n / 1024) ints of scratch; without it the scan allocates stream-ordered.

@@ -74,7 +74,7 @@ struct LenCache {
 };
 static thread_local std::vector<LenCache> g_len_cache;
 
-static int get_len(int L, FftLen* out) {
+int cached_len(int L, FftLen* out) {
     int dev = 0;
     HB_CUDA(cudaGetDevice(&dev));
     for (const auto& c : g_len_cache)
@@ -146,9 +146,9 @@ static int toep_run(const ToepGeom& t, const ToepArgs& a, float2* ws, cudaStream
     float2* W1 = ws;                                   // [N0][N1][L2][B]
     float2* W2 = ws + (size_t)N0 * N1 * L2 * B;        // [N0][L1][L2][B] (3-D only)
     FftLen f0, f1, f2;
-    HB_TRY(get_len(L2, &f2));
-    HB_TRY(get_len(L1, &f1));
-    if (t.dim == 3) HB_TRY(get_len(L0, &f0));
+    HB_TRY(cached_len(L2, &f2));
+    HB_TRY(cached_len(L1, &f1));
+    if (t.dim == 3) HB_TRY(cached_len(L0, &f0));
 
     const int64_t cpf = a.sense ? B / a.frames : 0;  // coils per frame (SENSE)
     // P1: axis 2, pad N2 -> L2, forward
@@ -410,17 +410,49 @@ int transform_toeplitz_kernel(int dim, const int64_t* kshape, const void* kin, v
 }
 
 int toeplitz_kernel_frames(int dim, const int64_t* kshape, int nframes, const int64_t* npts, const float* c0,
-                           const float* c1, const float* c2, const void* nudata, void* kout, int width, cudaStream_t s);
+                           const float* c1, const float* c2, const void* nudata, void* kout, int width, void* workspace,
+                           size_t workspace_bytes, cudaStream_t s);
 
 int toeplitz_kernel(int dim, const int64_t* kshape, int64_t M, const float* c0, const float* c1, const float* c2,
                     const void* nudata, void* kout, int width, cudaStream_t s) {
-    return toeplitz_kernel_frames(dim, kshape, 1, &M, c0, c1, c2, nudata, kout, width, s);
+    return toeplitz_kernel_frames(dim, kshape, 1, &M, c0, c1, c2, nudata, kout, width, nullptr, 0, s);
+}
+
+// Workspace of a kernel build: the type-1 plan's grids and per-point arrays, the padding passes' buffers, and a
+// bound on the partial planes of the dense segments (a segment of more than maxp candidates has at most twice
+// total / maxp parts, and at least two that share its planes). What does not
+// fit -- nothing, in 3-D at widths up to 7 -- is allocated.
+int toeplitz_kernel_workspace(int dim, const int64_t* kshape, int nframes, const int64_t* npts, int width, size_t* bytes) {
+    HB_REQUIRE(dim >= 2 && dim <= 3, HB_ERR_INVALID_ARG, "Toeplitz kernel must be 2-D or 3-D");
+    HB_REQUIRE(kshape && npts && bytes && nframes >= 1, HB_ERR_INVALID_ARG, "null argument");
+    size_t F = (size_t)nframes, M = 0, fine = 1, y = 1, r[3] = {1, 1, 1}, L[3] = {1, 1, 1};
+    for (int f = 0; f < nframes; ++f) M += npts[f] > 0 ? (size_t)npts[f] : 0;
+    for (int i = 0; i < dim; ++i) {
+        HB_REQUIRE(kshape[i] >= 4 && kshape[i] % 2 == 0, HB_ERR_SHAPE, "kernel dimensions must be even (2N)");
+        const int ax = 3 - dim + i;
+        L[ax] = (size_t)kshape[i];
+        r[ax] = L[ax] - 1;
+        const size_t nf = (size_t)plan_fine_size(kshape[i] - 1, dim, ax, width);
+        fine *= nf;
+        y *= i == 0 ? (dim == 3 ? r[ax] : nf) : nf;
+    }
+    const size_t keys = fine / 512 * 8 * F + 16;
+    size_t n = arena_piece(8 * fine * F) + arena_piece(8 * y * F);
+    n += 5 * arena_piece(4 * (keys + 1));                                    // bins, counts, offsets
+    n += 10 * arena_piece(4 * M) + arena_piece(8 * M);                       // coordinates, order, values
+    n += arena_piece(8 * F * r[0] * r[1] * r[2]) + arena_piece(8 * F * r[0] * r[1] * L[2]) + arena_piece(8 * F * r[0] * L[1] * L[2]);
+    // at most 6.5 candidates per point (segments of one tile)
+    const size_t parts = 2 * (13 * M / 2 / std::min<size_t>(4096, std::max<size_t>(512, M / 1184)) + 1);
+    n += arena_piece(parts * 24) + arena_piece(parts * (7 + 19) * 512) + (size_t)(1 << 20);
+    *bytes = n;
+    return HB_OK;
 }
 
 // The kernels of nframes frames: one frame-batched type-1 NUFFT over every frame's points, then
 // the zero-padding FFT passes over all frames' rows at once. kout is [nframes][2N..].
 int toeplitz_kernel_frames(int dim, const int64_t* kshape, int nframes, const int64_t* npts, const float* c0,
-                           const float* c1, const float* c2, const void* nudata, void* kout, int width, cudaStream_t s) {
+                           const float* c1, const float* c2, const void* nudata, void* kout, int width, void* workspace,
+                           size_t workspace_bytes, cudaStream_t s) {
     HB_REQUIRE(dim >= 2 && dim <= 3, HB_ERR_INVALID_ARG, "Toeplitz kernel must be 2-D or 3-D");
     HB_REQUIRE(kshape && npts && kout, HB_ERR_INVALID_ARG, "null argument");
     HB_REQUIRE(nframes >= 1, HB_ERR_INVALID_ARG, "nframes must be >= 1");
@@ -436,35 +468,38 @@ int toeplitz_kernel_frames(int dim, const int64_t* kshape, int nframes, const in
         Nimg *= kshape[i] / 2;
     }
     NufftPlan plan;
+    if (workspace) {
+        const size_t skip = (256 - ((uintptr_t)workspace & 255)) & 255;
+        if (workspace_bytes > skip) {
+            plan.arena = (char*)workspace + skip;
+            plan.arena_bytes = workspace_bytes - skip;
+            plan.arena_stream = s;
+        }
+    }
     int st = plan_make(&plan, 1, dim, nm, 1, 1, 1e-5f, width, 2.0, HB_METHOD_DEFAULT);
     float2 *red = nullptr, *b1 = nullptr, *b2 = nullptr;
     auto cleanup = [&]() {
+        plan_release(&plan, red);
+        plan_release(&plan, b1);
+        plan_release(&plan, b2);
         plan_free(&plan);
-        if (red) cudaFree(red);
-        if (b1) cudaFree(b1);
-        if (b2) cudaFree(b2);
     };
+    const int64_t r0 = L[0] > 1 ? L[0] - 1 : 1, r1 = L[1] - 1, r2 = L[2] - 1;
+    const size_t nred = (size_t)F * r0 * r1 * r2;
+    if (st == HB_OK) st = plan_alloc(&plan, (void**)&red, sizeof(float2) * nred, "toeplitz_kernel modes");
+    if (st == HB_OK) st = plan_alloc(&plan, (void**)&b1, sizeof(float2) * (size_t)F * r0 * r1 * L[2], "toeplitz_kernel axis 2");
+    if (st == HB_OK) st = plan_alloc(&plan, (void**)&b2, sizeof(float2) * (size_t)F * r0 * L[1] * L[2], "toeplitz_kernel axis 1");
     if (st != HB_OK) {
         cleanup();
         return st;
-    }
-    const int64_t r0 = L[0] > 1 ? L[0] - 1 : 1, r1 = L[1] - 1, r2 = L[2] - 1;
-    const size_t nred = (size_t)F * r0 * r1 * r2;
-    cudaError_t e = cudaMalloc(&red, sizeof(float2) * nred);
-    if (e == cudaSuccess) e = cudaMalloc(&b1, sizeof(float2) * (size_t)F * r0 * r1 * L[2]);
-    if (e == cudaSuccess) e = cudaMalloc(&b2, sizeof(float2) * (size_t)F * r0 * L[1] * L[2]);
-    if (e != cudaSuccess) {
-        cleanup();
-        set_error(std::string("toeplitz_kernel temporaries: ") + cudaGetErrorString(e));
-        return HB_ERR_ALLOC;
     }
     do {
         if ((st = plan_setpts_frames(&plan, nframes, npts, c0, c1, c2, s)) != HB_OK) break;
         if ((st = plan_execute(&plan, (const float2*)nudata, red, s)) != HB_OK) break;
         FftLen f0, f1, f2;
-        if ((st = get_len((int)L[2], &f2)) != HB_OK) break;
-        if ((st = get_len((int)L[1], &f1)) != HB_OK) break;
-        if (dim == 3 && (st = get_len((int)L[0], &f0)) != HB_OK) break;
+        if ((st = cached_len((int)L[2], &f2)) != HB_OK) break;
+        if ((st = cached_len((int)L[1], &f1)) != HB_OK) break;
+        if (dim == 3 && (st = cached_len((int)L[0], &f0)) != HB_OK) break;
         const float scale = (float)(1.0 / (double)Nimg);
         float2* K = (float2*)kout;
         // axis 2: [F r0 r1][r2] -> b1 [F r0 r1][L2]
@@ -489,7 +524,9 @@ int toeplitz_kernel_frames(int dim, const int64_t* kshape, int nframes, const in
             if ((st = launch_fft_pass(op, f0, F, E, (int)r0, 0, (int)L[0], 0, 0, 0, s, "toeplitz_kernel axis0")) != HB_OK)
                 break;
         }
-        if ((e = cudaStreamSynchronize(s)) != cudaSuccess) {
+        // what the plan allocated goes with it; a caller's workspace is stream-ordered
+        cudaError_t e = plan.arena ? cudaSuccess : cudaStreamSynchronize(s);
+        if (e != cudaSuccess) {
             set_error(std::string("toeplitz_kernel sync: ") + cudaGetErrorString(e));
             st = HB_ERR_CUDA;
         }

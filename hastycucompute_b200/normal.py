@@ -63,7 +63,7 @@ def build_toeplitz_kernel(coords: Sequence[torch.Tensor], shape: Sequence[int], 
         nud = torch.ones((1, M), dtype=torch.complex64, device=dev)
     else:
         nud = weights.reshape(1, M).to(torch.complex64).contiguous()
-    kernel = torch.zeros(tuple(2 * s for s in shape), dtype=torch.complex64, device=dev)
+    kernel = torch.empty(tuple(2 * s for s in shape), dtype=torch.complex64, device=dev)
     return toeplitz_kernel(coords, kernel, nud, kernel_width=kernel_width)
 
 

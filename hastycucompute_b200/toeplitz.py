@@ -56,10 +56,21 @@ def toeplitz_kernel(coords: Sequence[torch.Tensor], kernel: torch.Tensor, nudata
         raise ValueError("shape<1>() of nudata didn't match length of coord vectors")
     check_tensor(nd, "nudata", torch.complex64, (M,), kernel.device)
     cp = [ptr(c) for c in coords] + [C.c_void_p(None)] * (3 - dim)
-    with torch.cuda.device(kernel.device):
-        _lib.call("hb_toeplitz_kernel", dim, _lib.i64_array(kernel.shape), int(M), cp[0], cp[1], cp[2],
-                  ptr(nd), ptr(kernel), int(kernel_width), stream_ptr(kernel.device))
+    _build(kernel, tuple(kernel.shape), [int(M)], cp, nd, kernel_width)
     return kernel
+
+
+def _build(kernels: torch.Tensor, kshape: Sequence[int], counts: Sequence[int], cp, nd: torch.Tensor, kernel_width: int) -> None:
+    """hb_toeplitz_kernels_frames_ws with its temporaries from torch's caching allocator on the current stream:
+    the build allocates nothing itself and does not wait for the GPU at its end (allocating and freeing the
+    grids took two thirds of a 128^3 build)."""
+    dim, F, n = len(kshape), len(counts), C.c_size_t()
+    with torch.cuda.device(kernels.device):
+        _lib.call("hb_toeplitz_kernels_workspace_size", dim, _lib.i64_array(kshape), F, _lib.i64_array(counts), int(kernel_width),
+                  C.byref(n))
+        ws = torch.empty(int(n.value), dtype=torch.uint8, device=kernels.device)
+        _lib.call("hb_toeplitz_kernels_frames_ws", dim, _lib.i64_array(kshape), F, _lib.i64_array(counts), cp[0], cp[1], cp[2],
+                  ptr(nd), ptr(kernels), int(kernel_width), ptr(ws), int(n.value), stream_ptr(kernels.device))
 
 
 def toeplitz_kernels_frames(frame_coords: Sequence[Sequence[torch.Tensor]], kernels: torch.Tensor,
@@ -94,9 +105,7 @@ def toeplitz_kernels_frames(frame_coords: Sequence[Sequence[torch.Tensor]], kern
     cat = [torch.cat([fc[i] for fc in frame_coords]).contiguous() for i in range(dim)]
     nd = torch.cat(nds).contiguous()
     cp = [ptr(c) for c in cat] + [C.c_void_p(None)] * (3 - dim)
-    with torch.cuda.device(dev):
-        _lib.call("hb_toeplitz_kernels_frames", dim, _lib.i64_array(kernels.shape[1:]), F, _lib.i64_array(counts),
-                  cp[0], cp[1], cp[2], ptr(nd), ptr(kernels), int(kernel_width), stream_ptr(dev))
+    _build(kernels, tuple(kernels.shape[1:]), counts, cp, nd, kernel_width)
     return kernels
 
 

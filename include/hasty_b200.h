@@ -186,6 +186,18 @@ int hb_toeplitz_kernels_frames(int dim, const int64_t* kernel_shape, int nframes
                                const float* coord2, const void* nudata, void* kernel_out,
                                int kernel_width, void* stream);
 
+/* hb_toeplitz_kernels_frames with its temporaries in a caller's workspace of
+ * hb_toeplitz_kernels_workspace_size bytes: nothing is allocated (temporaries that do not fit are), and
+ * the kernel is complete in stream order, not when the call returns. The workspace is free again for
+ * later work on the same stream. */
+int hb_toeplitz_kernels_workspace_size(int dim, const int64_t* kernel_shape, int nframes,
+                                       const int64_t* npts, int kernel_width, size_t* bytes);
+int hb_toeplitz_kernels_frames_ws(int dim, const int64_t* kernel_shape, int nframes,
+                                  const int64_t* npts, const float* coord0, const float* coord1,
+                                  const float* coord2, const void* nudata, void* kernel_out,
+                                  int kernel_width, void* workspace, size_t workspace_bytes,
+                                  void* stream);
+
 /* transform_toeplitz_kernel, cpp/corelib/lib/fft/toeplitz.cppm:510-609: re-lays the
  * straight kernel ([2N..] c64, from hb_toeplitz_kernel) into the layout
  * hb_toeplitz_multiplication / hb_sense_normal read (same element count, c64), with the
