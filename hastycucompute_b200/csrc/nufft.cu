@@ -808,135 +808,210 @@ __global__ void __launch_bounds__(kSpreadThreads, (CC <= 8) ? 2 : 1)
 }
 
 // ---- interpolation with compile-time width ---------------------------------------------------
-// Lanes of a warp map to (point slot, transform). Each lane keeps its point's first cells and tap
-// weights in registers, so the W^d gathers of a point are independent loads the compiler can
-// keep in flight together.
+// Lanes of a warp map to (point slot, transform); a lane gathers its point's W^d cells. A CTA takes a run of
+// consecutive sorted points, so that its warps meet in L1.
+//
+// Bounds: the L1 data path (2 wavefronts per 32 loads of 8 bytes; 9.4 ms at 160^3 x 32, 6.1 M points, w = 6) and the
+// instructions issued. Misses do not bound it: 82 % L1 hits instead of 38 % gave no time. So what is not a load
+// or a multiply-add is kept small: sums are packed f32x2 multiply-adds on (re, im), a plane has one pointer, with
+// constant column offsets when the lanes hold all transforms, the taps of all axes are dealt to the slot's lanes at
+// once and shared rows are read 16 bytes at a time. Type 2 as above 22.7 -> 19.1 ms; 120x96x150 x 12, 1.5 M, w = 5: 2.99 -> 2.15;
+// 256^2 x 16, 0.2 M, w = 5: 0.180 -> 0.113; 90x110x75 x 5, 0.3 M, w = 5: 0.477 -> 0.395.
+// W floats of a shared row (16-byte aligned), four at a time
+template <int W>
+__device__ __forceinline__ void load_row(const float* row, float (&w)[W]) {
+#pragma unroll
+    for (int d = 0; d < W; d += 4) {
+        if (d + 4 <= W) {
+            const float4 q = *reinterpret_cast<const float4*>(row + d);
+            w[d] = q.x;
+            w[d + 1] = q.y;
+            w[d + 2] = q.z;
+            w[d + 3] = q.w;
+        } else {
+#pragma unroll
+            for (int e = d; e < W; ++e) w[e] = row[e];
+        }
+    }
+}
+
+// First cells and tap weights of a point: point_setup with the taps of all axes dealt to the slot's lanes at once
+// and the coefficients read four at a time (those above the degree are zero: the same values).
+template <int CC, int W>
+__device__ __forceinline__ void interp_setup(const GridArgs& a, const float* coef, int64_t s, bool valid, int lane_in_slot,
+                                             float* wts, int* i0) {
+    float sarg[3];
+#pragma unroll
+    for (int ax = 0; ax < 3; ++ax) {
+        i0[ax] = 0;
+        sarg[ax] = 0.f;
+        if (a.g.wa[ax] == 1) continue;
+        const float v = __fsub_rn(valid ? a.su[ax][s] : 0.f, a.kb.hw);
+        const int ic = (int)ceilf(v);
+        sarg[ax] = fmaf(2.f, __fsub_rn((float)ic, v), -1.f);
+        const int nf = a.g.nf[ax];
+        int iw = ic;
+        if (iw < 0) iw += nf;
+        if (iw >= nf) iw -= nf;
+        i0[ax] = iw;
+    }
+    auto tap = [&](int ax, int d, float sa) {
+        if (a.g.wa[ax] == 1) {
+            if (d == 0) wts[ax * kMaxWidth] = 1.f;
+            return;
+        }
+        float v;
+        if (a.kb.deg < 12) {
+            const float4* c = reinterpret_cast<const float4*>(coef + d * (kMaxDeg + 1));
+            const float4 c2 = c[2], c1 = c[1], c0 = c[0];
+            v = c2.w;
+            v = fmaf(v, sa, c2.z);
+            v = fmaf(v, sa, c2.y);
+            v = fmaf(v, sa, c2.x);
+            v = fmaf(v, sa, c1.w);
+            v = fmaf(v, sa, c1.z);
+            v = fmaf(v, sa, c1.y);
+            v = fmaf(v, sa, c1.x);
+            v = fmaf(v, sa, c0.w);
+            v = fmaf(v, sa, c0.z);
+            v = fmaf(v, sa, c0.y);
+            v = fmaf(v, sa, c0.x);
+        } else {
+            v = kb_tap(coef, a.kb.deg, d, sa);
+        }
+        wts[ax * kMaxWidth + d] = v;
+    };
+#pragma unroll 1
+    for (int t = lane_in_slot; t < 3 * W; t += CC) {
+        const int ax = t / W;
+        tap(ax, t - ax * W, ax == 0 ? sarg[0] : (ax == 1 ? sarg[1] : sarg[2]));
+    }
+}
+
+// The W x W cells of one z plane, RB rows of loads in flight at a time; CS is the column stride in transforms when it is
+// known (the loads then take constant offsets), 0 otherwise. Per row the sum over x, then the row's weight w_z w_y.
+template <int W, int RB, int CS>
+__device__ __forceinline__ void interp_plane(const float2* p, unsigned cs, unsigned rowstride, const f2_t (&wx)[W],
+                                             const float* wy, float wz, float& ar, float& ai) {
+    const unsigned cst = CS ? CS : cs;
+#pragma unroll
+    for (int y0 = 0; y0 < W; y0 += RB) {
+        f2_t v[RB][W];
+#pragma unroll
+        for (int r = 0; r < RB; ++r) {
+            if (y0 + r < W) {
+                const float2* q = p + (size_t)(y0 + r) * rowstride;
+#pragma unroll
+                for (int dx = 0; dx < W; ++dx) v[r][dx] = *reinterpret_cast<const f2_t*>(q + (size_t)dx * cst);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < RB; ++r) {
+            if (y0 + r < W) {
+                f2_t acc = f2_mul(wx[0], v[r][0]);
+#pragma unroll
+                for (int dx = 1; dx < W; ++dx) acc = f2_fma(wx[dx], v[r][dx], acc);
+                float rr, ri;
+                f2_unpack(acc, rr, ri);
+                const float wzy = wz * wy[y0 + r];
+                ar = fmaf(wzy, rr, ar);
+                ai = fmaf(wzy, ri, ai);
+            }
+        }
+    }
+}
+
+// Rows of a plane whose loads are in flight together, and the CTAs per SM that the registers are held to. One
+// transform: 32 points a warp and uncoalesced loads, which want the whole plane in flight (96^3, 0.5 M points, w = 6: 268 us
+// at 2 CTAs, 283 at 3). Two and four: half planes at 3 CTAs (4 transforms: 481 us, 511 at 2). From eight on
+// two rows at 4 CTAs (120x96x150 x 12, 1.5 M, w = 5: 2.15 ms, half planes at 3 CTAs 2.32, whole planes at 2 2.51), whole
+// planes where they are small (w <= 4), 3 CTAs where four would spill (w = 7, 8).
+template <int CC, int W>
+struct InterpShape {
+    static constexpr int RB = W > 8 ? 2 : CC == 1 ? (W <= 6 ? W : 4) : CC < 8 ? (W <= 6 ? (W + 1) / 2 : 4) : W <= 4 ? W : 2;
+    static constexpr int MB = W > 8 ? 1 : CC == 1 ? 2 : CC < 8 ? (W <= 6 ? 3 : 2) : W <= 6 ? 4 : 3;
+};
+
 template <int CC, int W, bool FR>
-__global__ void __launch_bounds__(kGridThreads) k_interp_w(const GridArgs a) {
-    extern __shared__ float sm[];
+__global__ void __launch_bounds__(kGridThreads, InterpShape<CC, W>::MB) k_interp_w(const GridArgs a, int run) {
+    extern __shared__ float4 interp_f4[];
     constexpr int NS = 32 / CC;
-    float* coef = sm;
-    float* wts_all = coef + kCoefFloats;
+    float* const coef = reinterpret_cast<float*>(interp_f4);
+    float* const wts_all = coef + kCoefFloats;
     const GridGeom& g = a.g;
     for (int i = threadIdx.x; i < kCoefFloats; i += blockDim.x) coef[i] = (&a.kb.coef[0][0])[i];
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int slot = lane / CC, coil = lane % CC;
-    float* wts = wts_all + (warp * NS + slot) * kSlotFloats;
-    const int64_t gwarp = (int64_t)blockIdx.x * kGridWarps + warp;
-    const int64_t nwarps = (int64_t)gridDim.x * kGridWarps;
+    float* const wts = wts_all + (warp * NS + slot) * kSlotFloats;
+    const int64_t run0 = (int64_t)blockIdx.x * run, run1 = min(run0 + run, g.M);
     const int nf0 = g.nf[0], nf1 = g.nf[1], nf2 = g.nf[2];
     const int wz = g.wa[0], wy = g.wa[1];
-    for (int64_t base = gwarp * NS; base < g.M; base += nwarps * NS) {
+    const unsigned rowstride = (unsigned)nf2 * (unsigned)g.C;
+    for (int64_t base = run0 + warp * NS; base < run1; base += kGridWarps * NS) {
         const int64_t s = base + slot;
-        const bool valid = s < g.M;
+        const bool valid = s < run1;
         int i0[3];
-        point_setup(a, coef, s, valid, coil, CC, wts, i0);
+        interp_setup<CC, W>(a, coef, s, valid, coil, wts, i0);
         __syncwarp();
         if (valid) {
-            // element offsets of the taps along axis 2 (x C transforms), 32-bit: a grid holds
-            // fewer than 2^32 complex values (checked when the plan is made)
-            unsigned colofs[W];
-            float wx[W];
-#pragma unroll
-            for (int d = 0; d < W; ++d) {
-                int v = i0[2] + d;
-                if (v >= nf2) v -= nf2;
-                colofs[d] = (unsigned)v * (unsigned)g.C;
-                wx[d] = wts[2 * kMaxWidth + d];
-            }
             const int pj = a.perm[s];
             // frames (FR): the grid block of the point's frame; one frame reads a.grid itself
             const float2* const gridf = FR ? a.grid + frame_of_point(a.foff, g.nfr, s) * g.fgrid : a.grid;
-            const unsigned rowstride = (unsigned)nf2 * (unsigned)g.C;
-            // Common case: the footprint wraps neither along axis 2 nor axis 1 and the lanes hold
-            // all C transforms, so a tap's column stride is the compile-time CC: one row pointer,
-            // W loads at constant offsets.
-            const bool slab_fast = (W <= 6) && g.C % CC == 0 && wy == W && i0[2] + W <= nf2 && i0[1] + W <= nf1;
-            const unsigned cs = (unsigned)g.C;  // column stride of a tap along axis 2
+            float wxs[W];
+            f2_t wx[W];
+            load_row<W>(wts + 2 * kMaxWidth, wxs);
+#pragma unroll
+            for (int d = 0; d < W; ++d) wx[d] = f2_dup(wxs[d]);
+            // the footprint wraps neither along axis 2 nor along axis 1: one pointer per plane
+            const bool inside = wy == W && i0[2] + W <= nf2 && i0[1] + W <= nf1;
             for (int cc0 = 0; cc0 < g.C; cc0 += CC) {
                 if (cc0 + coil >= g.C) break;
-                const float2* gridc = gridf + cc0 + coil;
+                const float2* const gridc = gridf + cc0 + coil;
                 float ar = 0.f, ai = 0.f;
-                for (int dz = 0; dz < wz; ++dz) {
-                    int gz = i0[0] + dz;
-                    if (gz >= nf0) gz -= nf0;
-                    const float wzv = wts[dz];
-                    if constexpr (W <= 6) {
-                        if (slab_fast) {
-                            const float2* p0 =
-                                gridc + (((unsigned)gz * (unsigned)nf1 + (unsigned)i0[1]) * (unsigned)nf2 + (unsigned)i0[2]) * cs;
-                            float2 v[W * W];
-#pragma unroll
-                            for (int dy = 0; dy < W; ++dy) {
-                                const float2* pr = p0 + (size_t)dy * rowstride;
-#pragma unroll
-                                for (int dx = 0; dx < W; ++dx) v[dy * W + dx] = pr[dx * (g.C == CC ? CC : cs)];
-                            }
-#pragma unroll
-                            for (int dy = 0; dy < W; ++dy) {
-                                float rr = 0.f, ri = 0.f;
-#pragma unroll
-                                for (int dx = 0; dx < W; ++dx) {
-                                    rr = fmaf(wx[dx], v[dy * W + dx].x, rr);
-                                    ri = fmaf(wx[dx], v[dy * W + dx].y, ri);
-                                }
-                                const float wzy = wzv * wts[kMaxWidth + dy];
-                                ar = fmaf(wzy, rr, ar);
-                                ai = fmaf(wzy, ri, ai);
-                            }
-                            continue;
-                        }
-                    }
-                    unsigned rowbase[W];
-#pragma unroll
-                    for (int dy = 0; dy < W; ++dy) {
-                        int gy = i0[1] + dy;
-                        if (gy >= nf1) gy -= nf1;
-                        rowbase[dy] = ((unsigned)gz * (unsigned)nf1 + (unsigned)gy) * rowstride;
-                    }
-                    if constexpr (W <= 6) {
-                        // issue the whole W x W slab of gathers before any multiply
-                        float2 v[W * W];
-#pragma unroll
-                        for (int dy = 0; dy < W; ++dy) {
-                            const float2* rowp = gridc + rowbase[dy];
-#pragma unroll
-                            for (int dx = 0; dx < W; ++dx)
-                                v[dy * W + dx] = dy < wy ? rowp[colofs[dx]] : make_float2(0.f, 0.f);
-                        }
-#pragma unroll
-                        for (int dy = 0; dy < W; ++dy) {
-                            // row partial sum with the axis-2 weights, then one multiply by the row weight
-                            float rr = 0.f, ri = 0.f;
-#pragma unroll
-                            for (int dx = 0; dx < W; ++dx) {
-                                rr = fmaf(wx[dx], v[dy * W + dx].x, rr);
-                                ri = fmaf(wx[dx], v[dy * W + dx].y, ri);
-                            }
-                            const float wzy = dy < wy ? wzv * wts[kMaxWidth + dy] : 0.f;
-                            ar = fmaf(wzy, rr, ar);
-                            ai = fmaf(wzy, ri, ai);
-                        }
+                if (inside) {
+                    // element offsets are 32-bit: a grid holds fewer than 2^32 complex values (checked
+                    // when the plan is made)
+                    auto plane = [&](int dz) {
+                        int gz = i0[0] + dz;
+                        if (gz >= nf0) gz -= nf0;
+                        return gridc + (((unsigned)gz * (unsigned)nf1 + (unsigned)i0[1]) * (unsigned)nf2 + (unsigned)i0[2]) * (unsigned)g.C;
+                    };
+                    if (g.C == CC) {
+#pragma unroll 1
+                        for (int dz = 0; dz < wz; ++dz)
+                            interp_plane<W, InterpShape<CC, W>::RB, CC>(plane(dz), CC, rowstride, wx, wts + kMaxWidth, wts[dz], ar, ai);
                     } else {
+#pragma unroll 1
+                        for (int dz = 0; dz < wz; ++dz)
+                            interp_plane<W, InterpShape<CC, W>::RB, 0>(plane(dz), (unsigned)g.C, rowstride, wx, wts + kMaxWidth, wts[dz], ar, ai);
+                    }
+                } else {
+                    unsigned colofs[W];
 #pragma unroll
-                        for (int dy = 0; dy < W; ++dy) {
-                            if (dy < wy) {
-                                const float wzy = wzv * wts[kMaxWidth + dy];
-                                const float2* rowp = gridc + rowbase[dy];
-                                float2 v[W];
+                    for (int d = 0; d < W; ++d) {
+                        int v = i0[2] + d;
+                        if (v >= nf2) v -= nf2;
+                        colofs[d] = (unsigned)v * (unsigned)g.C;
+                    }
+#pragma unroll 1
+                    for (int r = 0; r < wz * wy; ++r) {
+                        const int dz = wy == 1 ? r : r / W, dy = wy == 1 ? 0 : r - dz * W;
+                        int gz = i0[0] + dz, gy = i0[1] + dy;
+                        if (gz >= nf0) gz -= nf0;
+                        if (gy >= nf1) gy -= nf1;
+                        const float2* rowp = gridc + ((unsigned)gz * (unsigned)nf1 + (unsigned)gy) * rowstride;
+                        f2_t v[W];
 #pragma unroll
-                                for (int dx = 0; dx < W; ++dx) v[dx] = rowp[colofs[dx]];
-                                float rr = 0.f, ri = 0.f;
+                        for (int dx = 0; dx < W; ++dx) v[dx] = *reinterpret_cast<const f2_t*>(rowp + colofs[dx]);
+                        f2_t acc = f2_mul(wx[0], v[0]);
 #pragma unroll
-                                for (int dx = 0; dx < W; ++dx) {
-                                    rr = fmaf(wx[dx], v[dx].x, rr);
-                                    ri = fmaf(wx[dx], v[dx].y, ri);
-                                }
-                                ar = fmaf(wzy, rr, ar);
-                                ai = fmaf(wzy, ri, ai);
-                            }
-                        }
+                        for (int dx = 1; dx < W; ++dx) acc = f2_fma(wx[dx], v[dx], acc);
+                        float rr, ri;
+                        f2_unpack(acc, rr, ri);
+                        const float wzy = wts[dz] * wts[kMaxWidth + dy];
+                        ar = fmaf(wzy, rr, ar);
+                        ai = fmaf(wzy, ri, ai);
                     }
                 }
                 a.out[(int64_t)(cc0 + coil) * g.M + pj] = make_float2(ar, ai);
@@ -1628,16 +1703,20 @@ static int launch_spread_cc(const NufftPlan* p, const GridArgs& a, cudaStream_t 
 template <int CC, int W>
 static int launch_interp_w(const NufftPlan* p, const GridArgs& a, cudaStream_t s) {
     const int64_t per_block = (int64_t)kGridWarps * (32 / CC);
-    int64_t blocks = ceil_div(std::max<int64_t>(p->g.M, 1), per_block);
-    blocks = std::min<int64_t>(blocks, (int64_t)kNumSMs * 64);
+    // Sorted points of a CTA: up to four turns of its warps (more turns gain nothing up to 12 transforms, and at 160^3 x 32 cost
+    // 19.1 -> 20.7 ms a type 2 at eight: fewer planes of the grid stay in L2), fewer where that would leave less
+    // than 32 CTAs an SM (128^3 x 16, 64000 points in runs of 48 instead of 16: 1.27 -> 1.29 ms).
+    const int64_t turns = std::clamp<int64_t>(p->g.M / (per_block * kNumSMs * 32), 1, 4);
+    const int64_t run = per_block * turns;
+    const int64_t blocks = ceil_div(std::max<int64_t>(p->g.M, 1), run);
     const size_t smem = sizeof(float) * (kCoefFloats + (size_t)kGridWarps * (32 / CC) * kSlotFloats);
     TimedSection ts("interp", s);
     if (a.foff) {
         HB_CUDA(cudaFuncSetAttribute(k_interp_w<CC, W, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_interp_w<CC, W, true><<<(unsigned)blocks, kGridThreads, smem, s>>>(a);
+        k_interp_w<CC, W, true><<<(unsigned)blocks, kGridThreads, smem, s>>>(a, (int)run);
     } else {
         HB_CUDA(cudaFuncSetAttribute(k_interp_w<CC, W, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_interp_w<CC, W, false><<<(unsigned)blocks, kGridThreads, smem, s>>>(a);
+        k_interp_w<CC, W, false><<<(unsigned)blocks, kGridThreads, smem, s>>>(a, (int)run);
     }
     return check_launch("k_interp");
 }
