@@ -452,6 +452,11 @@ __device__ __forceinline__ c2 pair_tw(const PairCfg& c, int L, int t, int k1, co
     return c2_mul_tw<INV>(v, tw[at]);
 }
 
+// Full-length samples of the plain operators share the transpose's memory: step 1 reads and writes the L slots of a
+// pair's column set in place.
+template <class Op, int HM>
+constexpr bool kPairInPlace = !Op::kLoadLFast && !Op::kFusedK && ((HM & 4) != 0 || (HM & 3) == 2);
+
 // Step 1 for radix P: the thread's samples, P-point DFT, outer twiddles, into the transpose.
 template <int P, class Op, int HM, bool INV>
 __device__ __forceinline__ void pair_step1(const Op& op, const PairCfg& c, int L, int Q, const PairCols& k, int t, int cp,
@@ -482,6 +487,9 @@ __device__ __forceinline__ void pair_step1(const Op& op, const PairCfg& c, int L
         c2_dft_halfzero<P, INV>(v);
     else
         c2_dft<P, INV>(v);
+    // rotated slots: a lane overwrites samples of the other lanes of its t (eight lanes of one warp, all of them here),
+    // which must have read them first. Without rotation every lane writes the slots that it has read itself.
+    if constexpr (kPairInPlace<Op, HM> && Op::kStoreLFast) __syncwarp(0xffu << (threadIdx.x & 24));
 #pragma unroll
     for (int k1 = 0; k1 < P; ++k1) {
         if (k1 > 0 || (PH && (c.ph & 2))) v[k1] = PH ? pair_tw<INV>(c, L, t, k1, tw, v[k1]) : c2_mul_tw<INV>(v[k1], tw[t * k1]);
@@ -587,8 +595,8 @@ __device__ __forceinline__ void radix_switch(int r, F&& f) {
 // Persistent CTAs walk the jobs (row block, column block) with a stride of the grid; a reducing operator
 // takes all column blocks of a row block in turn. While a job is transformed the next one's samples are copied:
 // into their own buffer In, free once step 1 has read it (INPL false), or -- full-length samples --
-// into the transpose itself, free once step 2 has read it (INPL true: step 1 reads and writes the same
-// slots; half the shared memory, so more CTAs per SM).
+// into the transpose itself, free once step 2 has read it (INPL true: the eight lanes of a t read and write the
+// same slots in step 1; half the shared memory, so more CTAs per SM).
 template <class Op, int HM, bool INV, int RMIN, int RMAX, int PT, int QT, int MB, bool INPL>
 __global__ void __launch_bounds__((RMAX * kPairs + 31) / 32 * 32, MB) pair_kernel(const Op op, const PairCfg c) {
     const int P = PT ? PT : c.P, Q = QT ? QT : c.Q, L = PT ? PT * QT : c.L;
@@ -754,8 +762,7 @@ __global__ void __launch_bounds__((RMAX * kPairs + 31) / 32 * 32, MB) pair_kerne
 
 template <class Op, int HM, bool INV, int RMIN, int RMAX, int PT, int QT, int MB>
 int launch_pair_inst(const Op& op, PairCfg c, cudaStream_t s, const char* name) {
-    // full-length samples share the transpose's memory
-    constexpr bool INPL = !Op::kLoadLFast && !Op::kFusedK && ((HM & 4) != 0 || (HM & 3) == 2);
+    constexpr bool INPL = kPairInPlace<Op, HM>;
     auto kern = pair_kernel<Op, HM, INV, RMIN, RMAX, PT, QT, MB, INPL>;
     c.W = kCW;
     c.in_stride = c.Lin | 1;
