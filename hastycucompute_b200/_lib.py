@@ -22,6 +22,7 @@ STATUS_NAMES = {
     5: "HB_ERR_STATE",
     6: "HB_ERR_RANGE",
     7: "HB_ERR_WORKSPACE",
+    8: "HB_ERR_TIMEOUT",
 }
 
 # Every function the header declares, with (restype, argtypes).
@@ -40,6 +41,8 @@ SIGNATURES = {
     "hb_nufft_set_spread_kernel": (_i, [_vp, _i, _i]),
     "hb_nufft_set_interp_tuning": (_i, [_vp, _i]),
     "hb_nufft_set_interp_kernel": (_i, [_vp, _i]),
+    "hb_nufft_set_spread_wait": (_i, [_vp, _i]),
+    "hb_nufft_check": (_i, [_vp, _vp]),
     "hb_nufft_get_info": (_i, [_vp, _pi64, C.POINTER(_i), C.POINTER(_d), C.POINTER(_sz)]),
     "hb_toeplitz_kernel": (_i, [_i, _pi64, _i64, _vp, _vp, _vp, _vp, _vp, _i, _vp]),
     "hb_toeplitz_kernels_frames": (_i, [_i, _pi64, _i, _pi64, _vp, _vp, _vp, _vp, _vp, _i, _vp]),

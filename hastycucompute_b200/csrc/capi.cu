@@ -170,6 +170,26 @@ int hb_nufft_set_interp_kernel(hb_nufft_plan plan, int kind) {
     })
 }
 
+int hb_nufft_set_spread_wait(hb_nufft_plan plan, int tries) {
+    HB_GUARD({
+        if (!plan) {
+            hb::set_error("plan is null");
+            return HB_ERR_INVALID_ARG;
+        }
+        return hb::plan_set_spread_wait(&plan->p, tries);
+    })
+}
+
+int hb_nufft_check(hb_nufft_plan plan, void* stream) {
+    HB_GUARD({
+        if (!plan) {
+            hb::set_error("plan is null");
+            return HB_ERR_INVALID_ARG;
+        }
+        return hb::plan_check(&plan->p, as_stream(stream));
+    })
+}
+
 int hb_nufft_coord_grad(hb_nufft_plan plan, const void* modes, const void* h, float* grad, void* stream) {
     HB_GUARD({
         if (!plan) {

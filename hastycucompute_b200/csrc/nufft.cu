@@ -1287,7 +1287,7 @@ int plan_make(NufftPlan* p, int type, int dim, const int64_t* nmodes, int sign, 
     }
     p->nbins_cap = p->nbins * p->sub;
     HB_TRY(dev_alloc(p, (void**)&p->bin_start, sizeof(int) * (p->nbins_cap + 1), "bins"));
-    HB_TRY(dev_alloc(p, (void**)&p->d_err, sizeof(int), "error flag"));
+    HB_TRY(dev_alloc(p, (void**)&p->d_err, 2 * sizeof(int), "error flags"));
     return HB_OK;
 }
 
@@ -1330,7 +1330,8 @@ static WalkArgs walk_args(const NufftPlan* p) {
     w.n_parts = (int)p->n_parts;
     w.range = p->walk_range;
     w.scratch = p->dense_scratch;
-    w.err = p->d_err;
+    w.err = p->d_err + 1;
+    w.tries = p->walk_tries;
     return w;
 }
 
@@ -1354,6 +1355,26 @@ static int st_build_jobs(NufftPlan* p, cudaStream_t s) {
 
 int plan_setpts(NufftPlan* p, int64_t M, const float* c0, const float* c1, const float* c2, cudaStream_t s) {
     return plan_setpts_frames(p, 1, &M, c0, c1, c2, s);
+}
+
+// An execute's spreading gave up waiting: reported and cleared.
+static int report_spread_wait(NufftPlan* p, cudaStream_t s) {
+    HB_CUDA(cudaMemsetAsync(p->d_err + 1, 0, sizeof(int), s));
+    set_error("a wait inside the spreading kernel of an earlier execute ran out; its output holds NaN");
+    return HB_ERR_TIMEOUT;
+}
+
+int plan_check(NufftPlan* p, cudaStream_t s) {
+    int err = 0;
+    if (p->err_clear) HB_CUDA(cudaMemcpyAsync(&err, p->d_err + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
+    HB_CUDA(cudaStreamSynchronize(s));
+    return err ? report_spread_wait(p, s) : HB_OK;
+}
+
+int plan_set_spread_wait(NufftPlan* p, int tries) {
+    HB_REQUIRE(tries >= 0 && tries <= kWalkTries, HB_ERR_INVALID_ARG, "tries must be in [0, 2^20]");
+    p->walk_tries = tries;
+    return HB_OK;
 }
 
 int plan_setpts_frames(NufftPlan* p, int nframes, const int64_t* npts, const float* c0, const float* c1,
@@ -1457,11 +1478,12 @@ int plan_setpts_frames(NufftPlan* p, int nframes, const int64_t* npts, const flo
     do {
         cudaError_t e = cudaSuccess;
         if ((e = cudaMemsetAsync(count, 0, sizeof(int) * (nkeys + 1), s)) != cudaSuccess ||
-            (e = cudaMemsetAsync(p->d_err, 0, sizeof(int), s)) != cudaSuccess) {
+            (e = cudaMemsetAsync(p->d_err, 0, (p->err_clear ? 1 : 2) * sizeof(int), s)) != cudaSuccess) {
             set_error(std::string("setpts memset: ") + cudaGetErrorString(e));
             st = HB_ERR_CUDA;
             break;
         }
+        p->err_clear = true;
         if (M > 0) {
             FoldArgs fa{};
             for (int ax = 0; ax < 3; ++ax) {
@@ -1626,16 +1648,20 @@ int plan_setpts_frames(NufftPlan* p, int nframes, const int64_t* npts, const flo
         p->st_built = false;
         if (p->type == 2 && p->st && (st = st_build_jobs(p, s)) != HB_OK) break;
         {
-            int err = 0;
-            if ((e = cudaMemcpyAsync(&err, p->d_err, sizeof(int), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
+            int err[2] = {0, 0};
+            if ((e = cudaMemcpyAsync(err, p->d_err, sizeof(err), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
                 (e = cudaStreamSynchronize(s)) != cudaSuccess) {
                 set_error(std::string("setpts sync: ") + cudaGetErrorString(e));
                 st = HB_ERR_CUDA;
                 break;
             }
-            if (err) {
+            if (err[0]) {
                 set_error("setpts: non-finite coordinate");
                 st = HB_ERR_RANGE;
+                break;
+            }
+            if (err[1]) {
+                st = report_spread_wait(p, s);
                 break;
             }
         }

@@ -35,6 +35,8 @@ struct GridGeom {
     int64_t fgrid;    // fine grid values per frame (cells x C)
 };
 
+constexpr int kWalkTries = 1 << 20;  // of a wait inside k_spread_walk: two seconds
+
 struct NufftPlan {
     int type = 1;
     int sign = 1;
@@ -63,7 +65,8 @@ struct NufftPlan {
     int64_t extra_cap = 0;
     float2* extra_scratch = nullptr;
     size_t extra_scratch_cap = 0;  // bytes
-    int* d_err = nullptr;
+    int* d_err = nullptr;      // [0] non-finite coordinate in this setpts; [1] a spreading wait ran out (kept until reported)
+    bool err_clear = false;    // [1] has been cleared since the plan was made
     bool pts_set = false;
     // frames: grids are allocated for frames_cap frames; foff holds the current frames' point
     // offsets (device, g.nfr + 1 entries)
@@ -99,6 +102,7 @@ struct NufftPlan {
     bool walk_ok = false;
     int sub = 1;
     int walk_sp = 8, walk_ns = 1;
+    int walk_tries = kWalkTries;
     int2* walk_range = nullptr;
     int64_t walk_range_cap = 0;
     int interp_cc = 0;  // interpolation: transforms per lane group (0 = the spreading rule)
@@ -191,6 +195,9 @@ int plan_set_spread_tuning(NufftPlan* p, int maxp, int bz, int by, int bx);
 int plan_set_spread_kernel(NufftPlan* p, int kind, int transforms_per_cta);
 int plan_set_interp_tuning(NufftPlan* p, int transforms_per_group);
 int plan_set_interp_kernel(NufftPlan* p, int kind);
+int plan_set_spread_wait(NufftPlan* p, int tries);
+// waits for the stream; HB_ERR_TIMEOUT when a spreading wait of an earlier execute ran out (reported once)
+int plan_check(NufftPlan* p, cudaStream_t s);
 
 // Type-2 interpolation from staged regions of the fine grid (interp_st.cu). interp_st_jobs with
 // jobs == nullptr counts the jobs (per tile in cnt, offsets in off, total in *n_jobs; syncs s);

@@ -46,6 +46,7 @@ struct WalkArgs {
     int2* range;              // first and last first-cell of each part
     float2* scratch;          // [plane][64 cells][C]
     int* err;                 // set when a wait ran out (never with a correct kernel)
+    int tries;                // of a wait, up to 2 us each
 };
 
 constexpr int kWalkMaxCells = 32 + 6;  // first cells of a segment
@@ -106,10 +107,11 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* b) {
 __device__ __forceinline__ void mbar_arrive_copies(uint64_t* b) {
     asm volatile("cp.async.mbarrier.arrive.noinc.shared.b64 [%0];" ::"r"((unsigned)__cvta_generic_to_shared(b)) : "memory");
 }
-// waits for the phase of the given parity; false when it did not come (bounded)
-__device__ __forceinline__ bool mbar_wait(uint64_t* b, unsigned parity) {
+// Waits for the phase of the given parity; false when it did not come within `tries`. Lanes of a warp may differ, so
+// they vote on it before any of them leaves.
+__device__ __forceinline__ bool mbar_wait(uint64_t* b, unsigned parity, int tries) {
     const unsigned addr = (unsigned)__cvta_generic_to_shared(b);
-    for (int i = 0; i < (1 << 20); ++i) {
+    for (int i = 0; i < tries; ++i) {
         unsigned ok;
         asm volatile(
             "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared.b64 p, [%1], %2, %3;\nselp.u32 %0, 1, 0, p;\n}"
@@ -264,11 +266,11 @@ __global__ void __launch_bounds__(WalkShape<CC, W>::THREADS, WalkShape<CC, W>::M
 
     const int nch = (k_end - k_begin + S::CH - 1) / S::CH;
     const int cell0 = is_part ? cell_of(k_begin) : 0;  // the walk's first cell
-    // Stages chunk c, one thread per candidate; false when a wait ran out.
+    // Stages chunk c, one thread per candidate; false (for a whole warp) when a wait ran out.
     auto stage = [&](int c, int q) -> bool {
         const int b = c % S::RING;
         float* buf = ring + b * S::kBufF;
-        if (c >= S::RING && !mbar_wait(m_free + b, (c / S::RING - 1) & 1)) return false;
+        if (c >= S::RING && !__all_sync(0xffffffffu, mbar_wait(m_free + b, (c / S::RING - 1) & 1, w.tries))) return false;
         const int k = k_begin + c * S::CH + q;
         int pk = 0, cell = 0, pj = 0, ry = -16, rx = -16;  // past the end: reaches no block
         float fz = 0.f, fy = 0.f, fx = 0.f;
@@ -344,9 +346,9 @@ __global__ void __launch_bounds__(WalkShape<CC, W>::THREADS, WalkShape<CC, W>::M
 
     if (warp >= S::WARPS) {  // staging warps
         bool ok = true;
-        for (int c = 0; c < nch && ok; ++c) ok = __all_sync(0xffffffffu, stage(c, tid - S::WARPS * 32));
+        for (int c = 0; c < nch && ok; ++c) ok = stage(c, tid - S::WARPS * 32);
         cp_async_wait_all();
-        if (!ok && lane == 0) atomicExch(w.err, 2);
+        if (!ok && lane == 0) atomicExch(w.err, 1);
         return;
     }
 
@@ -442,7 +444,7 @@ __global__ void __launch_bounds__(WalkShape<CC, W>::THREADS, WalkShape<CC, W>::M
                 return;
             }
             const int b = c % S::RING;
-            ok = __all_sync(0xffffffffu, mbar_wait(m_full + b, (c / S::RING) & 1));  // a warp stays together
+            ok = __all_sync(0xffffffffu, mbar_wait(m_full + b, (c / S::RING) & 1, w.tries));  // a warp stays together
             if (!ok) {
                 e = kDone;
                 return;
@@ -499,7 +501,20 @@ __global__ void __launch_bounds__(WalkShape<CC, W>::THREADS, WalkShape<CC, W>::M
             out += plane_stride;
         }
     }
-    if (!ok && lane == 0) atomicExch(w.err, 2);
+    if (!ok) {
+        // a wait ran out, so the sums miss candidates: no value of this warp's cells may pass for a result
+        for (int r = first; r < stop; ++r) {
+            float2* const p = out + (int64_t)(r - cur) * plane_stride;
+            const float2 nan = make_float2(__int_as_float(0x7fffffff), __int_as_float(0x7fffffff));
+            if constexpr (S::CELLS) {
+                for (int k = 0; k < S::K; ++k)
+                    if (k < g.C) p[k] = nan;
+            } else if (coil_ok) {
+                p[0] = p[g.C] = p[row_stride] = p[row_stride + g.C] = nan;
+            }
+        }
+        if (lane == 0) atomicExch(w.err, 1);
+    }
 }
 
 // Adds the parts of the dense segments: CTA blockIdx.x is part e.y of e.z of segment e.x and takes that share of

@@ -525,11 +525,7 @@ int toeplitz_kernel_frames(int dim, const int64_t* kshape, int nframes, const in
                 break;
         }
         // what the plan allocated goes with it; a caller's workspace is stream-ordered
-        cudaError_t e = plan.arena ? cudaSuccess : cudaStreamSynchronize(s);
-        if (e != cudaSuccess) {
-            set_error(std::string("toeplitz_kernel sync: ") + cudaGetErrorString(e));
-            st = HB_ERR_CUDA;
-        }
+        if (!plan.arena) st = plan_check(&plan, s);
     } while (0);
     cleanup();
     return st;

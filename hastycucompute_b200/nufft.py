@@ -210,6 +210,16 @@ class NufftPlan:
         code = {"auto": 0, "cells": 1, "transforms": 2}[kind]
         _lib.call("hb_nufft_set_spread_kernel", self._h, code, int(transforms_per_cta))
 
+    def set_spread_wait(self, tries: int) -> None:
+        """Limit of a wait inside the 3-D spreading kernel, in tries of up to 2 us (0 .. 2^20, the default)."""
+        _lib.call("hb_nufft_set_spread_wait", self._h, int(tries))
+
+    def check(self) -> None:
+        """Waits for the current stream and raises HastyError (HB_ERR_TIMEOUT) if a wait inside the spreading kernel
+        of an earlier execute ran out; that execute's output holds NaN. setpts raises it as well."""
+        with torch.cuda.device(self.device):
+            _lib.call("hb_nufft_check", self._h, stream_ptr(self.device))
+
     def set_interp_tuning(self, transforms_per_group: int = 0) -> None:
         """Interpolation (type 2): transforms per lane group (points per warp = 32 / that; 0 =
         automatic). All choices compute the same sums."""

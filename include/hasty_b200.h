@@ -43,6 +43,7 @@ extern "C" {
 #define HB_ERR_STATE        5  /* call order violated (execute before setpts, ...)      */
 #define HB_ERR_RANGE        6  /* non-finite coordinate met during setpts                */
 #define HB_ERR_WORKSPACE    7  /* caller-provided workspace smaller than required        */
+#define HB_ERR_TIMEOUT      8  /* a bounded wait inside a kernel ran out                 */
 
 /* ---- enums (values identical to the reference) --------------------------------------- */
 /* nufft_type, cpp/corelib/lib/fft/nufft.cppm:42-48 */
@@ -129,6 +130,13 @@ int hb_nufft_set_spread_tuning(hb_nufft_plan plan, int max_candidates, int block
 #define HB_SPREAD_CELLS      1
 #define HB_SPREAD_TRANSFORMS 2
 int hb_nufft_set_spread_kernel(hb_nufft_plan plan, int kind, int transforms_per_cta);
+
+/* The 3-D spreading kernel's warps hand candidates to one another through bounded waits (tries of
+ * up to 2 us, 0 .. 2^20, 2^20 when never set). An execute whose wait ran out, which no correct run
+ * does, puts NaN into its output; hb_nufft_check waits for `stream` and returns HB_ERR_TIMEOUT for
+ * it once, as does the plan's next setpts. */
+int hb_nufft_set_spread_wait(hb_nufft_plan plan, int tries);
+int hb_nufft_check(hb_nufft_plan plan, void* stream);
 
 /* Interpolation of a type-2 plan (no counterpart in the reference): the transforms one group of
  * lanes gathers per point (1, 2, 4, 8, 16 or 32; 0 = automatic), i.e. 32 / that many points per
