@@ -502,16 +502,15 @@ __global__ void __launch_bounds__(WalkShape<CC, W>::THREADS, WalkShape<CC, W>::M
         }
     }
     if (!ok) {
-        // a wait ran out, so the sums miss candidates: no value of this warp's cells may pass for a result
-        for (int r = first; r < stop; ++r) {
-            float2* const p = out + (int64_t)(r - cur) * plane_stride;
-            const float2 nan = make_float2(__int_as_float(0x7fffffff), __int_as_float(0x7fffffff));
-            if constexpr (S::CELLS) {
-                for (int k = 0; k < S::K; ++k)
-                    if (k < g.C) p[k] = nan;
-            } else if (coil_ok) {
-                p[0] = p[g.C] = p[row_stride] = p[row_stride + g.C] = nan;
-            }
+        // a wait ran out, so the sums miss candidates: NaN in the last plane stored (the FFT passes take it to every
+        // output; poisoning all planes kept `first` alive through the walk, 2 % of a type 1 of 12 transforms)
+        float2* const p = out - (cur - stop + 1) * (int64_t)plane_stride;
+        const float2 nan = make_float2(__int_as_float(0x7fffffff), __int_as_float(0x7fffffff));
+        if constexpr (S::CELLS) {
+            for (int k = 0; k < S::K; ++k)
+                if (k < g.C) p[k] = nan;
+        } else if (coil_ok) {
+            p[0] = p[g.C] = p[row_stride] = p[row_stride + g.C] = nan;
         }
         if (lane == 0) atomicExch(w.err, 1);
     }
