@@ -73,4 +73,19 @@ inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 constexpr int kNumSMs = 148;  // B200
 
+// Lets a kernel whose dynamic shared memory differs from launch to launch have `smem` bytes. The limit belongs to
+// the kernel, not to the launch, and is shared by all host threads: it is always set to the most a CTA can have, so no
+// thread lowers it between another one's call and its launch. static_bytes: bound on the kernel's own __shared__ arrays.
+constexpr size_t kMaxSmem = 227 * 1024;
+template <class K>
+int allow_smem(K* kern, size_t smem, const char* what, size_t static_bytes = 0) {
+    const size_t most = kMaxSmem - static_bytes;
+    if (smem > most) {
+        set_error(std::string(what) + ": needs " + std::to_string(smem) + " bytes of shared memory, a CTA has " + std::to_string(most));
+        return HB_ERR_CUDA;
+    }
+    HB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+    return HB_OK;
+}
+
 }  // namespace hb

@@ -442,12 +442,7 @@ template <class Op>
 int launch_pass(const Op& op, const PassCfg& c, size_t extra_bytes, cudaStream_t s, const char* name) {
     const size_t smem = pass_smem_bytes(c, extra_bytes);
     static_assert(kPassThreads == 256, "");
-    cudaError_t e = cudaFuncSetAttribute(pass_kernel<Op>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-
-    if (e != cudaSuccess) {
-        set_error(std::string(name) + ": cudaFuncSetAttribute failed: " + cudaGetErrorString(e));
-        return HB_ERR_CUDA;
-    }
+    HB_TRY(allow_smem(pass_kernel<Op>, smem, name));
     const int64_t n_ab = ceil_div(c.A, c.A_blk);
     const int64_t blocks = Op::kChunkLoop ? n_ab : n_ab * c.n_eb;
     if (blocks <= 0) return HB_OK;

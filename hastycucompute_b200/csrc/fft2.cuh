@@ -681,9 +681,10 @@ struct HalfIO<Op, std::void_t<decltype(Op::kHalfIO)>> {
 template <int P, int Q, class Op, int HM, bool PF>
 int launch_pass2_inst(const Op& op, const PassCfg& c, size_t smem, int64_t blocks, cudaStream_t s, const char* name) {
     auto kern = pass2_kernel<P, Q, Op, HM, PF>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    HB_TRY(allow_smem(kern, smem, name));
+    cudaError_t e = cudaSuccess;
     // the staging passes want every CTA they can fit; plain passes keep the default L1 split
-    if (e == cudaSuccess && (Op::kFusedK || Op::kSenseReduce || PF))
+    if (Op::kFusedK || Op::kSenseReduce || PF)
         e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) {
         set_error(std::string(name) + ": cudaFuncSetAttribute failed: " + cudaGetErrorString(e));

@@ -778,8 +778,8 @@ int launch_pair_inst(const Op& op, PairCfg c, cudaStream_t s, const char* name) 
     if (Op::kFusedK) smem += (size_t)c.n_k * c.L * sizeof(float2);
     if (Op::kSenseReduce) smem += (size_t)(c.Lout * kPairs + kCW * c.s_stride) * sizeof(float2);
     const int threads = (std::max(c.P, c.Q) * kPairs + 31) / 32 * 32;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    HB_TRY(allow_smem(kern, smem, name));
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     int per_sm = 0;
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
     if (e != cudaSuccess) {

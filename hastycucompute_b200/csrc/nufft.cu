@@ -1710,7 +1710,7 @@ static int launch_spread_cc(const NufftPlan* p, const GridArgs& a, cudaStream_t 
         return HB_OK;
     }
     const size_t smem = sizeof(float) * ((size_t)2 * cells * CC + kCoefFloats + (size_t)kGridWarps * (32 / CC) * kSlotFloats);
-    HB_CUDA(cudaFuncSetAttribute(k_spread<CC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    HB_TRY(allow_smem(k_spread<CC>, smem, "k_spread", 1024));
     {
         TimedSection ts("spread", s);
         k_spread<CC><<<(unsigned)p->nbins, kGridThreads, smem, s>>>(a, 0);
