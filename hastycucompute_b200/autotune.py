@@ -3,9 +3,11 @@ subproblem for a given problem by timing type-1 plans on the device, and the int
 groups by timing type-2 plans, and caches the choices as JSON.
 
 Spreading search space (all exact, all give the same result up to float rounding):
-- the kernel: transforms on the lanes (each thread owns 4 rows x 8 cells of one transform; dense
-  tiles are spread in parts whose partial tiles a second kernel sums) or cells on the lanes (each
-  thread owns one cell; dense tiles as extra subproblems);
+- the kernel: "transforms", in 3-D at widths 4 .. 7 the kernel that walks along z (each lane group owns 2 x 2
+  cells over the planes of a footprint; dense segments are spread in parts whose planes a second kernel
+  sums), else 4 rows x 8 cells of one transform per thread; or "cells" (each thread owns one cell; dense
+  tiles as extra subproblems). Below five transforms, where "transforms" cannot be asked for, 3-D plans
+  walk by default, so "auto" is timed there;
 - for cells on the lanes, the 32-cell block each warp owns inside a spread tile: 3-D tiles are
   8x8x8, so any (bz, by, bx) with bz*by*bx = 32 and each edge dividing 8; 2-D tiles are 16x32;
 - points per subproblem (when a tile is dense enough to split): 256 .. 8192.
@@ -13,7 +15,8 @@ Spreading search space (all exact, all give the same result up to float rounding
 Interpolation search space: the transforms a lane group gathers per point (32, 16, 8 or 4 lanes;
 all give bit-identical results).
 
-Cache key: dimensionality, modes, transforms, kernel width, number of points and a coarse
+Cache key: the revision of the kernels (older choices were timed against kernels that are gone),
+dimensionality, modes, transforms, kernel width, number of points and a coarse
 density signature of the trajectory (quartiles of |k|), so the same trajectory family reuses the
 choice. Cache file: $HASTY_B200_TUNE_CACHE or ~/.cache/hastycucompute_b200/spread_tuning.json.
 """
@@ -34,6 +37,10 @@ MAXP = [1024, 2048, 4096, 8192]
 MAXP_TRANSFORMS = [256, 512, 1024, 2048, 4096]
 
 
+# counts up whenever a spreading or interpolation kernel, or what "auto" means, changes
+KERNEL_REVISION = 2
+
+
 def cache_path() -> Path:
     p = os.environ.get("HASTY_B200_TUNE_CACHE")
     if p:
@@ -46,7 +53,7 @@ def _key(nmodes, ntransf, width, coords) -> str:
     q = torch.quantile(r[:: max(1, r.numel() // 100000)], torch.tensor([0.25, 0.5, 0.75], device=r.device))
     sig = ",".join(f"{v:.2f}" for v in q.tolist())
     M = coords[0].shape[0]
-    return f"d{len(nmodes)}|n{'x'.join(map(str, nmodes))}|t{ntransf}|w{width}|m{M // 1000}k|q{sig}"
+    return f"r{KERNEL_REVISION}|d{len(nmodes)}|n{'x'.join(map(str, nmodes))}|t{ntransf}|w{width}|m{M // 1000}k|q{sig}"
 
 
 def _load() -> dict:
@@ -65,6 +72,13 @@ def _store(d: dict) -> None:
     p.write_text(json.dumps(d, indent=1, sort_keys=True))
 
 
+def spread_candidates(nmodes: Sequence[int], ntransf: int) -> list:
+    """The (kernel, block, max_candidates) that tune_spread times (a plan refuses those it has no kernel for)."""
+    blocks = BLOCKS_3D if len(nmodes) == 3 else BLOCKS_2D
+    wide = "auto" if len(nmodes) == 3 and ntransf < 5 else "transforms"
+    return [(wide, blocks[0], m) for m in MAXP_TRANSFORMS] + [("cells", b, m) for b in blocks for m in MAXP]
+
+
 def tune_spread(nmodes: Sequence[int], ntransf: int, coords: Sequence[torch.Tensor], kernel_width: int,
                 reps: int = 3, use_cache: bool = True, candidates: Optional[list] = None) -> dict:
     """Times type-1 executes over the search space; returns {"kernel", "block", "max_candidates",
@@ -76,10 +90,8 @@ def tune_spread(nmodes: Sequence[int], ntransf: int, coords: Sequence[torch.Tens
     if key in cache:
         return dict(cache[key], cached=True)
     dev = coords[0].device
-    blocks = BLOCKS_3D if len(nmodes) == 3 else BLOCKS_2D
     if candidates is None:
-        candidates = [("transforms", blocks[0], m) for m in MAXP_TRANSFORMS]
-        candidates += [("cells", b, m) for b in blocks for m in MAXP]
+        candidates = spread_candidates(nmodes, ntransf)
     M = coords[0].shape[0]
     data = torch.randn((ntransf, M), dtype=torch.complex64, device=dev)
     out = torch.empty((ntransf, *nmodes), dtype=torch.complex64, device=dev)
