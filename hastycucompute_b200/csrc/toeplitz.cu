@@ -524,8 +524,8 @@ int toeplitz_kernel_frames(int dim, const int64_t* kshape, int nframes, const in
             if ((st = launch_fft_pass(op, f0, F, E, (int)r0, 0, (int)L[0], 0, 0, 0, s, "toeplitz_kernel axis0")) != HB_OK)
                 break;
         }
-        // what the plan allocated goes with it; a caller's workspace is stream-ordered
-        if (!plan.arena) st = plan_check(&plan, s);
+        // the kernel is complete, on any stream, when the call returns
+        st = plan_check(&plan, s);
     } while (0);
     cleanup();
     return st;

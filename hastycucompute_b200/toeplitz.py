@@ -40,7 +40,8 @@ def toeplitz_kernel(coords: Sequence[torch.Tensor], kernel: torch.Tensor, nudata
     """toeplitz_kernel (nufft.cppm:386-441): fills ``kernel`` ([2N..], complex64) in place.
 
     ``nudata`` is [1, M] (or [M]) complex64 weights (ones, or a density compensation).
-    ``kernel_width`` <= 0 derives the width from tol 1e-5 (w = 6 at upsampling 2).
+    ``kernel_width`` <= 0 derives the width from tol 1e-5 (w = 6 at upsampling 2). The call returns when the
+    kernel is complete, so it may be used on any stream.
     """
     dim = kernel.dim()
     if dim not in (2, 3):
@@ -61,9 +62,8 @@ def toeplitz_kernel(coords: Sequence[torch.Tensor], kernel: torch.Tensor, nudata
 
 
 def _build(kernels: torch.Tensor, kshape: Sequence[int], counts: Sequence[int], cp, nd: torch.Tensor, kernel_width: int) -> None:
-    """hb_toeplitz_kernels_frames_ws with its temporaries from torch's caching allocator on the current stream:
-    the build allocates nothing itself and does not wait for the GPU at its end (allocating and freeing the
-    grids took two thirds of a 128^3 build)."""
+    """hb_toeplitz_kernels_frames_ws with its temporaries from torch's caching allocator on the current stream: the
+    build allocates nothing itself (allocating and freeing the grids took two thirds of a 128^3 build)."""
     dim, F, n = len(kshape), len(counts), C.c_size_t()
     with torch.cuda.device(kernels.device):
         _lib.call("hb_toeplitz_kernels_workspace_size", dim, _lib.i64_array(kshape), F, _lib.i64_array(counts), int(kernel_width),

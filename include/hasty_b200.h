@@ -195,9 +195,7 @@ int hb_toeplitz_kernels_frames(int dim, const int64_t* kernel_shape, int nframes
                                int kernel_width, void* stream);
 
 /* hb_toeplitz_kernels_frames with its temporaries in a caller's workspace of
- * hb_toeplitz_kernels_workspace_size bytes: nothing is allocated (temporaries that do not fit are), and
- * the kernel is complete in stream order, not when the call returns. The workspace is free again for
- * later work on the same stream. */
+ * hb_toeplitz_kernels_workspace_size bytes: nothing is allocated but temporaries that do not fit. */
 int hb_toeplitz_kernels_workspace_size(int dim, const int64_t* kernel_shape, int nframes,
                                        const int64_t* npts, int kernel_width, size_t* bytes);
 int hb_toeplitz_kernels_frames_ws(int dim, const int64_t* kernel_shape, int nframes,
