@@ -268,13 +268,16 @@ constexpr int kRadixMax = 26;
 constexpr bool pair_radix(int r) {
     return (r >= 8 && r <= 16) || r == 18 || r == 20 || r == 21 || r == 22 || r == 24 || r == 25 || r == 26;
 }
+// the instance of a split (run-time radices), by its larger radix: the smallest radix it has a step for
+constexpr int pair_rmin(int larger) { return larger <= 16 ? 8 : larger <= 20 ? 9 : 10; }
 
-// (P, Q) of length L, the most even split into two radices of the set; {0, 0} where there is none. Of the two
+// (P, Q) of length L, the most even split into two radices of the set that one instance has; {0, 0} where there is
+// none (189 = 9 x 21: the instance of 21 begins at 10). Of the two
 // orders the one whose P (input_side) or Q is divisible by 4, else by 2: the side that a pass pads or crops.
-inline void pair_split(int L, bool input_side, int* P, int* Q) {
+constexpr void pair_split(int L, bool input_side, int* P, int* Q) {
     *P = *Q = 0;
     for (int hi = 8; hi <= kRadixMax; ++hi) {
-        if (!pair_radix(hi) || L % hi != 0 || L / hi > hi || !pair_radix(L / hi)) continue;
+        if (!pair_radix(hi) || L % hi != 0 || L / hi > hi || !pair_radix(L / hi) || L / hi < pair_rmin(hi)) continue;
         const int lo = L / hi;
         auto rank = [](int r) { return r % 4 == 0 ? 2 : r % 2 == 0 ? 1 : 0; };
         const bool lo_first = input_side ? rank(lo) >= rank(hi) : rank(hi) >= rank(lo);
@@ -283,6 +286,20 @@ inline void pair_split(int L, bool input_side, int* P, int* Q) {
         return;
     }
 }
+// every split is a product of two radices that its instance has
+constexpr bool pair_splits_served() {
+    for (int L = 1; L <= kRadixMax * kRadixMax; ++L) {
+        for (int side = 0; side < 2; ++side) {
+            int P = 0, Q = 0;
+            pair_split(L, side != 0, &P, &Q);
+            if (P == 0) continue;
+            const int larger = P > Q ? P : Q, smaller = P > Q ? Q : P;
+            if (P * Q != L || !pair_radix(P) || !pair_radix(Q) || smaller < pair_rmin(larger)) return false;
+        }
+    }
+    return true;
+}
+static_assert(pair_splits_served(), "a radix without a step would leave its outputs unwritten");
 
 struct PairCfg {
     int P, Q, L;
@@ -801,9 +818,9 @@ int launch_pair_dir(const Op& op, const PairCfg& c, cudaStream_t s, const char* 
     if (c.P == 8 && c.Q == 16) return launch_pair_inst<Op, HM, INV, 8, 16, 8, 16, 4>(op, c, s, name);
     if (c.P == 16 && c.Q == 16) return launch_pair_inst<Op, HM, INV, 16, 16, 16, 16, 4>(op, c, s, name);
     if (c.P == 16 && c.Q == 20) return launch_pair_inst<Op, HM, INV, 16, 20, 16, 20, 3>(op, c, s, name);
-    if (r <= 16) return launch_pair_inst<Op, HM, INV, 8, 16, 0, 0, 4>(op, c, s, name);
-    if (r <= 20) return launch_pair_inst<Op, HM, INV, 9, 20, 0, 0, 3>(op, c, s, name);
-    return launch_pair_inst<Op, HM, INV, 10, kRadixMax, 0, 0, 2>(op, c, s, name);
+    if (r <= 16) return launch_pair_inst<Op, HM, INV, pair_rmin(16), 16, 0, 0, 4>(op, c, s, name);
+    if (r <= 20) return launch_pair_inst<Op, HM, INV, pair_rmin(20), 20, 0, 0, 3>(op, c, s, name);
+    return launch_pair_inst<Op, HM, INV, pair_rmin(kRadixMax), kRadixMax, 0, 0, 2>(op, c, s, name);
 }
 
 inline bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
