@@ -441,8 +441,9 @@ int toeplitz_kernel_workspace(int dim, const int64_t* kshape, int nframes, const
     n += 5 * arena_piece(4 * (keys + 1));                                    // bins, counts, offsets
     n += 10 * arena_piece(4 * M) + arena_piece(8 * M);                       // coordinates, order, values
     n += arena_piece(8 * F * r[0] * r[1] * r[2]) + arena_piece(8 * F * r[0] * r[1] * L[2]) + arena_piece(8 * F * r[0] * L[1] * L[2]);
-    // at most 6.5 candidates per point (segments of one tile)
-    const size_t parts = 2 * (13 * M / 2 / std::min<size_t>(4096, std::max<size_t>(512, M / 1184)) + 1);
+    // a point is a candidate of at most eight segments: four columns, and two segments of each when its first z cell
+    // is one of the W - 1 below the next segment
+    const size_t parts = 2 * (8 * M / std::min<size_t>(4096, std::max<size_t>(512, M / 1184)) + 1);
     n += arena_piece(parts * 24) + arena_piece(parts * (7 + 19) * 512) + (size_t)(1 << 20);
     *bytes = n;
     return HB_OK;
