@@ -429,6 +429,7 @@ int toeplitz_kernel_workspace(int dim, const int64_t* kshape, int nframes, const
     for (int f = 0; f < nframes; ++f) M += npts[f] > 0 ? (size_t)npts[f] : 0;
     for (int i = 0; i < dim; ++i) {
         HB_REQUIRE(kshape[i] >= 4 && kshape[i] % 2 == 0, HB_ERR_SHAPE, "kernel dimensions must be even (2N)");
+        HB_REQUIRE(kshape[i] - 1 <= (1 << 20), HB_ERR_INVALID_ARG, "nmodes out of range");
         const int ax = 3 - dim + i;
         L[ax] = (size_t)kshape[i];
         r[ax] = L[ax] - 1;
@@ -436,6 +437,9 @@ int toeplitz_kernel_workspace(int dim, const int64_t* kshape, int nframes, const
         fine *= nf;
         y *= i == 0 ? (dim == 3 ? r[ax] : nf) : nf;
     }
+    // refused here as the build refuses it, before a caller allocates for it
+    HB_REQUIRE(fine < ((size_t)1 << 32), HB_ERR_INVALID_ARG, "fine grid must hold fewer than 2^32 values");
+    HB_REQUIRE(M < 0x7fffffff, HB_ERR_INVALID_ARG, "M must be in [0, 2^31)");
     const size_t keys = fine / 512 * 8 * F + 16;
     size_t n = arena_piece(8 * fine * F) + arena_piece(8 * y * F);
     n += 5 * arena_piece(4 * (keys + 1));                                    // bins, counts, offsets

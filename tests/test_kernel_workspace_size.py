@@ -23,3 +23,15 @@ def test_workspace_holds_the_dense_parts(w, maxp):
     segments = 8 * M // (maxp + 1)
     need = segments * (2 * (16 + 8) + (32 + w - 1 + 2 * w) * 64 * 8) + 44 * M
     assert _size((64, 64, 64), M, w)[1] - _size((64, 64, 64), 0, w)[1] >= need
+
+
+@pytest.mark.parametrize("shape,M", [((900, 900, 900), 10), ((1 << 20, 4), 10), ((16, 16), (1 << 31) - 1)])
+def test_refuses_what_the_build_refuses(shape, M):
+    """A fine grid of 2^32 cells, more than 2^20 modes and 2^31 points are argument errors of a build, so its caller
+    must not be sent to allocate a workspace for them first."""
+    assert _size(shape, M, 6)[0] == 1
+
+
+@pytest.mark.parametrize("shape,M", [((400, 400, 400), 10), ((1 << 19, 4), 10), ((16, 16), (1 << 31) - 2)])
+def test_takes_what_the_build_takes(shape, M):
+    assert _size(shape, M, 6)[0] == 0
