@@ -16,7 +16,13 @@
 //
 // P and Q are run-time values: the steps are compiled once per radix and chosen by a uniform
 // switch, so one kernel serves every length instead of one instance per length. Larger radices need
-// more registers, so there are three instances: radices up to 16, up to 20 and up to 26.
+// more registers, so there are three such instances: radices up to 16, up to 20 and up to 26. The lengths 64, 128,
+// 256 and 320 have instances with their radices as constants (launch_pair_dir).
+//
+// What bounds it at 320 points: not one unit but latency, with three CTAs of five warps an SM (128 registers). The
+// fused Toeplitz pass (160^3, 8 coils: 0.87 ms) has DRAM at 32 %, the FMA pipe at 47 %, issue slots at 50 % and the
+// shared-memory data path at 50 %; its warps wait for fixed latencies, barriers and shared memory. The plain
+// passes stand at 66 % of DRAM, the first and the last one at 47 and 42 %.
 //
 // Against the shared-memory Stockham kernel that served these lengths before (B200): the SENSE normal
 // operator at 88 x 104 x 110, 6 coils, 2.47 -> 0.53 ms; type 1 at 120 x 96 x 150, 12 transforms, 5.93 ->
@@ -906,8 +912,8 @@ int launch_pair_pass(const Op& op, const FftLen& f, int64_t A, int64_t E, int Li
     }
 }
 
-// Runs the pass kernel for the length: column pairs where L splits into two radices of 8 to 26 points (and is
-// none of the lengths with an instance of their own), else launch_wide_pass.
+// Runs the pass kernel for the length: column pairs where L splits into two radices of 8 to 26 points and a side is
+// padded or cropped, else launch_wide_pass.
 // `extra_per_row` is the kSenseReduce accumulator size per outer row (bytes).
 template <class Op>
 int launch_fft_pass(const Op& op, const FftLen& f, int64_t A, int64_t E, int Lin, int in_shift, int Lout, int out_shift,

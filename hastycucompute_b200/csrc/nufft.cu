@@ -808,15 +808,6 @@ __global__ void __launch_bounds__(kSpreadThreads, (CC <= 8) ? 2 : 1)
 }
 
 // ---- interpolation with compile-time width ---------------------------------------------------
-// Lanes of a warp map to (point slot, transform); a lane gathers its point's W^d cells. A CTA takes a run of
-// consecutive sorted points, so that its warps meet in L1.
-//
-// Bounds: the L1 data path (2 wavefronts per 32 loads of 8 bytes; 9.4 ms at 160^3 x 32, 6.1 M points, w = 6) and the
-// instructions issued. Misses do not bound it: 82 % L1 hits instead of 38 % gave no time. So what is not a load
-// or a multiply-add is kept small: sums are packed f32x2 multiply-adds on (re, im), a plane has one pointer, with
-// constant column offsets when the lanes hold all transforms, the taps of all axes are dealt to the slot's lanes at
-// once and shared rows are read 16 bytes at a time. Type 2 as above 22.7 -> 19.1 ms; 120x96x150 x 12, 1.5 M, w = 5: 2.99 -> 2.15;
-// 256^2 x 16, 0.2 M, w = 5: 0.180 -> 0.113; 90x110x75 x 5, 0.3 M, w = 5: 0.477 -> 0.395.
 // W floats of a shared row (16-byte aligned), four at a time
 template <int W>
 __device__ __forceinline__ void load_row(const float* row, float (&w)[W]) {
@@ -932,6 +923,15 @@ struct InterpShape {
     static constexpr int MB = W > 8 ? 1 : CC == 1 ? 2 : CC < 8 ? (W <= 6 ? 3 : 2) : W <= 6 ? 4 : 3;
 };
 
+// Lanes of a warp map to (point slot, transform); a lane gathers its point's W^d cells. A CTA takes a run of
+// consecutive sorted points, so that its warps meet in L1.
+//
+// Bounds: the L1 data path (2 wavefronts per 32 loads of 8 bytes; 9.4 ms at 160^3 x 32, 6.1 M points, w = 6), 85 % busy at
+// 96^3 x 32, 786 k radial points (issue slots 48 %). Misses do not bound it: 82 % L1 hits instead of 38 % gave no time. What is not a load
+// or a multiply-add is kept small: sums are packed f32x2 multiply-adds on (re, im), a plane has one pointer, with
+// constant column offsets when the lanes hold all transforms, the taps of all axes are dealt to the slot's lanes at
+// once and shared rows are read 16 bytes at a time. Type 2 as above 22.7 -> 19.1 ms; 120x96x150 x 12, 1.5 M, w = 5: 2.99 -> 2.15;
+// 256^2 x 16, 0.2 M, w = 5: 0.180 -> 0.113; 90x110x75 x 5, 0.3 M, w = 5: 0.477 -> 0.395.
 template <int CC, int W, bool FR>
 __global__ void __launch_bounds__(kGridThreads, InterpShape<CC, W>::MB) k_interp_w(const GridArgs a, int run) {
     extern __shared__ float4 interp_f4[];

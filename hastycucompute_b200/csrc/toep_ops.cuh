@@ -113,8 +113,8 @@ using OpToepInSense = OpToepInSenseT<false>;
 
 // The Toeplitz passes along the middle axis: zero-padding N -> 2N (forward) and cropping
 // 2N -> N (inverse), both at offset 0.
-// (Prefetching measured slower for both at 160^3 x 32 coils: P2 1.48 vs 1.26 ms, P4 1.36 vs 1.16 ms,
-// two or three CTAs per SM against four.)
+// (kPrefetch is of the single-column kernel, which serves 512 and 640 points: there it measured slower for both, two
+// or three CTAs per SM against four. The pair passes always copy the next job's samples ahead.)
 struct OpStridedPad : OpStrided {
     static constexpr int kHalfIO = 1;
 };

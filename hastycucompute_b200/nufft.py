@@ -202,9 +202,10 @@ class NufftPlan:
         _lib.call("hb_nufft_set_spread_tuning", self._h, int(max_candidates), *b)
 
     def set_spread_kernel(self, kind: str = "auto", transforms_per_cta: int = 0) -> None:
-        """Spreading kernel (before setpts): "auto", "cells" (one cell per lane) or "transforms"
-        (transforms on the lanes), and for the latter the transforms one CTA spreads (8, 16, 32;
-        0 = automatic). All compute the same sums."""
+        """Spreading kernel (before setpts): "cells" (one cell per lane), "transforms" (transforms on the lanes, five
+        or more; 3-D plans of widths 4..7 walk along z) or "auto" ("transforms" where the plan allows it; 3-D plans
+        of widths 4..7 walk with fewer transforms too), and the transforms one CTA spreads (8, 16, 32; 0 =
+        automatic). All compute the same sums."""
         if self.M is not None:
             raise RuntimeError("set the spreading kernel before setpts")
         code = {"auto": 0, "cells": 1, "transforms": 2}[kind]

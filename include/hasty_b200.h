@@ -112,20 +112,21 @@ int hb_nufft_setpts_frames(hb_nufft_plan plan, int nframes, const int64_t* npts,
 int hb_nufft_execute(hb_nufft_plan plan, const void* in, void* out, void* stream);
 
 /* Spreading knobs (no counterpart in the reference; set by the autotuner, before setpts): points
- * per spread subproblem (32..65536; when never set, setpts picks a power of two in 512..4096 from
- * the number of points) and the cell block a warp owns inside a spread tile (32 cells; default
+ * per spread subproblem (32..65536; when never set, setpts picks a power of two in 256..4096, from
+ * 512 where the plan walks, by the number of points) and the cell block a warp owns inside a spread tile (32 cells; default
  * 2x4x4 in 3-D, 1x4x8 in 2-D; power-of-two edges dividing the tile edge, unit axes 1). */
 int hb_nufft_set_spread_tuning(hb_nufft_plan plan, int max_candidates, int block_z, int block_y,
                                int block_x);
 
 /* Spreading kernel of a type-1 plan, before its setpts (no counterpart in the reference, whose
  * spreading method is cufinufft's GM / GM_SORT / SM choice, fft/nufft.cppm:119-139):
- * HB_SPREAD_AUTO (transforms on the lanes when the plan allows it: 8^3 or 16x32 tiles, widths
- * 4..8, 5 or more transforms, two or more tiles per axis), HB_SPREAD_CELLS (one cell per lane,
- * any plan), HB_SPREAD_TRANSFORMS (transforms on the lanes; HB_ERR_INVALID_ARG where the plan
- * does not allow it). transforms_per_cta (8, 16 or 32; 0 = automatic) sets how many transforms
- * one CTA of the transforms kernel spreads; larger transform counts run as several CTAs per tile.
- * Every choice computes the same sums. */
+ * HB_SPREAD_AUTO, HB_SPREAD_CELLS (one cell per lane, any plan) or HB_SPREAD_TRANSFORMS (transforms
+ * on the lanes: 8^3 or 16x32 tiles, widths 4..8, 5 or more transforms, two or more tiles per axis;
+ * HB_ERR_INVALID_ARG where the plan does not allow it). AUTO is TRANSFORMS where the plan allows
+ * it; 3-D plans of widths 4..7 walk along z under both, and under AUTO with fewer transforms too.
+ * transforms_per_cta (8, 16 or 32; 0 = automatic) sets how many transforms one CTA spreads with five
+ * or more; larger counts run as several CTAs per tile or column. Every choice computes the same
+ * sums. */
 #define HB_SPREAD_AUTO       0
 #define HB_SPREAD_CELLS      1
 #define HB_SPREAD_TRANSFORMS 2
