@@ -15,7 +15,7 @@
 // weights that are staged twice over, so no register moves are needed: 24 + 6 packed operations of two cycles each
 // at W = 6, of about 185 cycles that a visit takes per sub-core. No unit is full (96^3 x 32, 786 k radial points: issue
 // slots 51 %, FMA pipe 46 %, shared-memory data path 40 %): 20 warps an SM do not cover the latency of the
-// loads and of the multiply-adds. 160^3 x 32, 6.1 M points, w = 6: 12.3 ms, the tile kernel 20.1.
+// loads and of the multiply-adds. 160^3 x 32, 6.1 M points, w = 6: 12.5 ms, the tile kernel 20.1.
 //
 // Candidates are staged in chunks through a ring of three buffers by warps of their own, one thread per
 // candidate: it finds the candidate, tests whether its footprint reaches the column, and writes its
@@ -25,8 +25,8 @@
 // third of the time. A spreading warp first lists its candidates of a chunk, then visits the list.
 //
 // Segments with more than maxp candidates are spread in parts, one CTA each, into partial planes in
-// scratch; k_walk_reduce adds a segment's parts in part order. No atomics; every cell is written once
-// and the order of every sum is fixed for sorted points.
+// scratch; k_walk_reduce adds a segment's parts in part order. No atomics, and the order of every sum is fixed for
+// sorted points.
 #pragma once
 
 #include <algorithm>
@@ -52,6 +52,14 @@ struct WalkArgs {
 };
 
 constexpr int kWalkMaxCells = 32 + 6;  // first cells of a segment
+// Visits after which a warp puts its sums away into their planes (and adds to them there): a sum of n equal terms
+// rounds the same way at every step and drifts by up to n / 4 eps, and the points of a z cell at the centre of a
+// trajectory are much alike. Error against FP64 gridding of a smooth image's samples, without putting away, with runs of
+// 128 and of 64 visits (times of a type 1): 160^3 x 32, 6.1 M cones, w = 6: 3.5e-6, 3.9e-7, 1.6e-7 (17.2, 17.3,
+// 17.5 ms; the tile kernel 7.3e-7); 64^3 x 8, 131 k radial, w = 4: 1.0e-6, 2.0e-7, 1.4e-7 (256, 263, 263 us; the
+// tile kernel 1.4e-7); one transform 128^3, 2.1 M radial, w = 4: 2.2e-6, 4.6e-7, 1.9e-7 (0.92 ms each; the
+// cell kernel 1.1e-6).
+constexpr int kWalkRun = 64;
 
 // CC >= 8: the lanes hold transforms (groups of CC, 2 x 2 cells each). CC = 1, 2, 4: the lanes hold cells (a warp
 // 4 x 8 of the column's 8 x 8) and every thread all CC transforms of its cell.
@@ -434,6 +442,8 @@ __global__ void __launch_bounds__(WalkShape<CC, W>::THREADS, WalkShape<CC, W>::M
     bool ok = true;
     int c = -1;
     unsigned at = 0, e = kEnd;
+    // visits since the last plane was stored or the sums were put away | slots with sums in `out` << 16
+    unsigned run = 0;
     // this warp's candidates of the next chunk that has any: record address | first cell << 24
     auto next_list = [&]() {
         do {
@@ -469,38 +479,94 @@ __global__ void __launch_bounds__(WalkShape<CC, W>::THREADS, WalkShape<CC, W>::M
             __syncwarp();
             at = list_at;
             e = lds32(at);
+            run += nh;
         } while (e == kEnd);
     };
-    // one turn of the loop per W cells: in its d-th part the finished plane is the one in slot d
-    while (cur < stop) {
+    // adds to the plane's sums in `out`, j planes above `cur`, those in slot `sl`
+    auto put = [&](int j, int sl) {
+        float2* const p = out + (int64_t)j * plane_stride;
+        const bool add = (run >> (16 + sl)) & 1u;
+        if constexpr (S::CELLS) {
 #pragma unroll
-        for (int d = 0; d < W; ++d) {
-            for (;;) {
-                while ((int)(e >> 24) == cur) {
-                    const unsigned rec = e & 0xffffffu;
-                    at += 4;
-                    e = lds32(at);
-                    visit(rec);
+            for (int k = 0; k < S::K; ++k)
+                if (k < g.C) {
+                    f2_t* q = reinterpret_cast<f2_t*>(p + k);
+                    *q = add ? f2_add(acc[sl][k], *q) : acc[sl][k];
                 }
-                if (e != kEnd) break;
-                next_list();
-            }
-            if (cur >= first && cur < stop) {
-                if constexpr (S::CELLS) {
+        } else if (coil_ok) {
 #pragma unroll
-                    for (int k = 0; k < S::K; ++k)
-                        if (k < g.C) *reinterpret_cast<f2_t*>(out + k) = acc[d][k];
-                } else if (coil_ok) {
-                    *reinterpret_cast<f2_t*>(out) = acc[d][0];
-                    *reinterpret_cast<f2_t*>(out + g.C) = acc[d][1];
-                    *reinterpret_cast<f2_t*>(out + row_stride) = acc[d][2];
-                    *reinterpret_cast<f2_t*>(out + row_stride + g.C) = acc[d][3];
+            for (int k = 0; k < 4; ++k) {
+                f2_t* q = reinterpret_cast<f2_t*>(p + (k >> 1) * row_stride + (k & 1) * g.C);
+                *q = add ? f2_add(acc[sl][k], *q) : acc[sl][k];
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < S::K; ++k) acc[sl][k] = 0ull;
+    };
+    // Visits the candidates of first cell `cur`, whose plane is in slot D, and stores the plane; false when the list
+    // ends first.
+    auto walk_cell = [&](auto dc) -> bool {
+        constexpr int D = decltype(dc)::value;
+        while ((int)(e >> 24) == cur) {
+            const unsigned rec = e & 0xffffffu;
+            at += 4;
+            e = lds32(at);
+            visit(rec);
+        }
+        if (e == kEnd) return false;
+        if (cur >= first && cur < stop) put(0, D);
+#pragma unroll
+        for (int k = 0; k < S::K; ++k) acc[D][k] = 0ull;
+        run &= ~(0xffffu | 0x10000u << D);
+        ++cur;
+        out += plane_stride;
+        return true;
+    };
+    // the next list, with plane `cur` in slot d; before it the sums are put away after a long run
+    auto refill = [&](int d) {
+        if ((run & 0xffffu) >= (unsigned)kWalkRun) {
+#pragma unroll
+            for (int sl = 0; sl < W; ++sl) {
+                const int j = sl < d ? sl - d + W : sl - d;
+                if (cur + j >= first && cur + j < stop) {
+                    put(j, sl);
+                    run |= 0x10000u << sl;
                 }
             }
-#pragma unroll
-            for (int k = 0; k < S::K; ++k) acc[d][k] = 0ull;
-            ++cur;
-            out += plane_stride;
+            run &= ~0xffffu;
+        }
+        next_list();
+    };
+    // W cells a turn. With 32 transforms refill is compiled into every slot's loop; with fewer, where a list is shorter,
+    // once, and a switch leads back to the slot (spreading, 160^3 x 32: 11.7 ms, by the switch 12.9; 120x96x150 x 12:
+    // 1.22 ms, by the switch 1.13).
+    if constexpr (CC == 32) {
+        while (cur < stop) {
+            static_for<W>([&](auto dc) {
+                while (!walk_cell(dc)) refill(decltype(dc)::value);
+            });
+        }
+    } else {
+        int d = 0;
+        while (cur < stop) {
+            switch (d) {  // out of it with d < W where a list ended
+#define HB_WALK_SLOT(n)                                                \
+    case n:                                                            \
+        if constexpr (n < W) {                                         \
+            if (!walk_cell(std::integral_constant<int, n>{})) {        \
+                d = n;                                                 \
+                break;                                                 \
+            }                                                          \
+        }                                                              \
+        [[fallthrough]];
+                HB_WALK_SLOT(0) HB_WALK_SLOT(1) HB_WALK_SLOT(2) HB_WALK_SLOT(3) HB_WALK_SLOT(4) HB_WALK_SLOT(5) HB_WALK_SLOT(6)
+#undef HB_WALK_SLOT
+                default: d = W;
+            }
+            if (d == W)
+                d = 0;
+            else
+                refill(d);
         }
     }
     if (!ok) {
@@ -552,8 +618,13 @@ __global__ void __launch_bounds__(256) k_walk_reduce(const GridArgs a, const Wal
         const int64_t b0 = max(i0, p * PE) - p * PE, b1 = min(i1, (p + 1) * PE) - p * PE;
         const float2* src = w.scratch + ((int64_t)e.w + r) * PE;
         for (int64_t i = b0 + threadIdx.x; i < b1; i += blockDim.x) {
-            float2 sum = make_float2(0.f, 0.f);
-            for (int s = s0; s < s1; ++s) sum = cadd(sum, src[(int64_t)s * W * PE + i]);
+            double re = 0., im = 0.;  // (parts alike, some hundred at the centre of a radial trajectory)
+            for (int s = s0; s < s1; ++s) {
+                const float2 v = src[(int64_t)s * W * PE + i];
+                re += v.x;
+                im += v.y;
+            }
+            const float2 sum = make_float2((float)re, (float)im);
             const int cell = (int)(i / g.C), c = (int)(i - (int64_t)cell * g.C);
             gridf[(((int64_t)(z0 + p) * g.nf[1] + ty * 8 + (cell >> 3)) * g.nf[2] + tx * 8 + (cell & 7)) * g.C + c] = sum;
         }
