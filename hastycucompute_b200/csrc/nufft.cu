@@ -1230,7 +1230,7 @@ int plan_make(NufftPlan* p, int type, int dim, const int64_t* nmodes, int sign, 
     // lanes-on-transforms spreading: 8^3 (3-D) or 16x32 (2-D) tiles, widths 4..8, more than four
     // transforms, and at least two tiles along every non-unit axis (so no footprint wraps onto its
     // own tile). 3-D widths 4..7 walk along z, for any number of transforms, in 0.25 - 0.95 of the tile kernels'
-    // time at every size tried (160^3, 32 transforms, 6.1 M points, w = 6: 20.1 -> 12.4 ms; 128^3 x 16, 2 M
+    // time at every size tried (160^3, 32 transforms, 6.1 M points, w = 6: 20.1 -> 12.6 ms; 128^3 x 16, 2 M
     // points, w = 4: 3.35 -> 2.11; 64^3 x 32, 0.5 M, w = 7: 2.43 -> 2.24; 64^3 x 8, 131 k, w = 4: 0.26 ->
     // 0.16; 150^3 x 6, 40 k, w = 6: 0.55 -> 0.42; one transform 128^3, 2 M, w = 4: 2.86 -> 0.68; four 64^3,
     // 0.3 M, w = 5: 0.78 -> 0.33). At w = 8 the walk's 64 registers of cells spill (64^3 x 32, 0.5 M: 2.99 ->

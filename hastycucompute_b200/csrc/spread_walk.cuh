@@ -14,8 +14,8 @@
 // A visit is packed f32x2 arithmetic on (re, im): w_x v, w_y w_x v, then W multiply-adds per cell with
 // weights that are staged twice over, so no register moves are needed: 24 + 6 packed operations of two cycles each
 // at W = 6, of about 185 cycles that a visit takes per sub-core. No unit is full (96^3 x 32, 786 k radial points: issue
-// slots 51 %, FMA pipe 46 %, shared-memory data path 40 %): 20 warps an SM do not cover the latency of the
-// loads and of the multiply-adds. 160^3 x 32, 6.1 M points, w = 6: 12.5 ms, the tile kernel 20.1.
+// slots 50 %, FMA pipe 42 %, shared-memory data path 39 %): 20 warps an SM do not cover the latency of the
+// loads and of the multiply-adds. 160^3 x 32, 6.1 M points, w = 6: 12.6 ms, the tile kernel 20.1.
 //
 // Candidates are staged in chunks through a ring of three buffers by warps of their own, one thread per
 // candidate: it finds the candidate, tests whether its footprint reaches the column, and writes its
